@@ -1735,6 +1735,76 @@ __device__ __forceinline__ float waf_vflux<float>(float s_k1, float dtrdz, float
   return (0.5f * s_k1) * fmaf(-zphi, d, x1 + x0);
 }
 
+// The contracting builds (MOLOCH_FLUX_LIMITER) evaluate the FP64 WAF value in
+// flux form, without the slope ratio.  With d the difference across the face
+// and num the upwind one, phi d = is d + (zamu - is) L where
+//   L = superbee(num / d) d = sign(d) max(0, min(2 min(a, b), max(a, b))),
+//   a = sign(d) num, b = |d|
+// (the superbee limiter, P. K. Sweby, SIAM J. Numer. Anal. 21, 1984, times the
+// denominator of its argument), so half the WAF value is
+// x_upwind - 0.5 (zamu - is) L: no division, no guard against a small
+// denominator (for |d| < kMinden the two forms differ by less than
+// 4 kMinden), and with the velocity-only factors shared by a thread's fields
+// two FP64 operations a face instead of about 25.  GB300 has two FP64 lanes
+// an SM, and these kernels were bound by them (81-84 % busy, two thirds of
+// the FP64 step); minimum, maximum, doubling and sign run on the integer
+// pipe.  Where d is not finite the value is NaN, as in the quotient form.
+// Per step at 256 x 256 x 60: vertical 14.9 -> 4.2 ms, horizontal 18.0 -> 4.9
+// (tiles) or 4.2 ms (strips).  FP32 keeps the quotient form: its kernels wait
+// on memory (1.69 -> 1.63 and 1.76 -> 1.70 ms per step at 512 x 512 x 60 with
+// the flux form), and w, a small difference of large terms, moves by 1e-3 of
+// itself with any change of an FP32 rounding.
+#if defined(MOLOCH_FLUX_LIMITER)
+template <class T> constexpr bool kFluxForm = sizeof(T) == 8;
+#else
+template <class T> constexpr bool kFluxForm = false;
+#endif
+__device__ __forceinline__ double limited(double num, double d) {
+  typedef unsigned long long u64;
+  const u64 top = 0x8000000000000000ull;
+  const u64 db = (u64)__double_as_longlong(d), sg = db & top;
+  const u64 b = db ^ sg, a = (u64)__double_as_longlong(num) ^ sg;
+  const bool lt = a < b;  // non-negative doubles order as their bits; a < 0 is caught below
+  const u64 mn = lt ? a : b, mx = lt ? b : a;
+  const u64 two = mn >= (1ull << 52) ? mn + (1ull << 52) : mn;  // 2 mn (subnormals stay: below 2^-1022)
+  u64 l = two < mx ? two : mx;
+  if (a & top) l = 0ull;
+  if (b >= 0x7ff0000000000000ull) l = 0x7ff8000000000000ull;  // NaN where d is not finite
+  return __longlong_as_double((long long)(l ^ sg));
+}
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+// Velocity-only terms of a face: whether the positive direction is upwind
+// and 0.5 (zamu - is), zamu = vel dt
+template <class T>
+struct Face {
+  bool pos;
+  T hz;
+};
+template <class T>
+__device__ __forceinline__ Face<T> face_of(bool pos, T vel, T dt) {
+  return {pos, fma_rn(vel, mul_rn(T(0.5), dt), pos ? T(-0.5) : T(0.5))};
+}
+// half the WAF value at a face: d the difference across it (ahead minus
+// behind, or either order as long as npos and nneg, the differences across
+// the neighbouring faces behind and ahead, are in the same), xpos and xneg
+// the values behind and ahead
+template <class T>
+__device__ __forceinline__ T waf_half(const Face<T>& f, T d, T npos, T nneg, T xpos, T xneg) {
+  return fma_rn(-f.hz, limited(f.pos ? npos : nneg, d), f.pos ? xpos : xneg);
+}
+// new value of a cell: x + cb vb - ca va + (ca - cb) old, with vb, va half
+// the WAF values of the faces behind and ahead and cb, ca their velocities
+// times the metric terms
+template <class T>
+__device__ __forceinline__ T waf_update(T x, T cb, T vb, T ca, T va, T cdv, T old) {
+  return fma_rn(cdv, old, fma_rn(-ca, va, fma_rn(cb, vb, x)));
+}
+
 // One thread per column and F fields (F = 1, 2, 5 or 10: the tuned
 // View::vfields).  Both passes stream k in registers: pass 1 yields wz1(t)
 // at step t, pass 2 consumes it two levels later, so the intermediate field
@@ -1795,6 +1865,62 @@ __device__ __forceinline__ void b_waf_vertical_g(const View<T>& d, const int g, 
       return x;
     }
   };
+  if constexpr (kFluxForm<T>) {
+    // Flux form: the windows hold the two values a face takes and the
+    // differences across it and its neighbours, each formed once.  Pass 1 at
+    // step t: xb, xc = x(t), x(t+1), dx, ex = x(t-1)-x(t), x(t)-x(t+1); pass 2
+    // at m = t-2: y1, y2, y3 = wz1(m .. m+2), dy, ey likewise.
+    T xb[F], xc[F], dx[F], ex[F], y1[F], y2[F], y3[F], dy[F], ey[F];
+    T h1[F], h2[F];  // half WAF values of the faces above levels t and m
+#pragma unroll
+    for (int u = 0; u < F; ++u) {
+      xb[u] = xval(u, 0); xc[u] = kz > 1 ? xval(u, 1) : xb[u];
+      dx[u] = T(0); ex[u] = sub_rn(xb[u], xc[u]);
+      y1[u] = T(0); y2[u] = T(0); y3[u] = T(0); dy[u] = T(0); ey[u] = T(0);
+      h1[u] = T(0); h2[u] = T(0);
+    }
+    T sB = T(0), sC = s[c];                       // s(t-1), s(t)
+    T uA = T(0), uB = T(0), dA = T(0), dB = T(0);  // s(k) wafu(k), s(k+1) wafd(k) at k = t-2, t-1
+    auto step = [&](const int t, auto fast) {
+      constexpr bool FAST = decltype(fast)::value;
+      T uC = T(0), dC = T(0), sD = T(0);
+      const int m = t - 2;
+      if (FAST || t <= kz) {
+        sD = s[c + (unsigned)t * pl];
+        uC = mul_rn(sC, wafu[c + (unsigned)(t - 1) * pl]);
+        dC = mul_rn(sD, wafd[c + (unsigned)(t - 1) * pl]);
+      }
+      const Face<T> f1 = face_of(sD >= T(0), sD, dtrdz), f2 = face_of(sB >= T(0), sB, dtrdz);
+      const T v1 = sub_rn(uC, dC), v2 = sub_rn(uA, dA);
+#pragma unroll
+      for (int u = 0; u < F; ++u) {
+        T w1 = y3[u];
+        if (FAST || t <= kz) {
+          const T xd = (FAST || t + 2 <= kz) ? xval(u, t + 1) : xc[u];  // x(min(t+2, kz))
+          const T d3 = sub_rn(xc[u], xd);
+          const T h = (FAST || t <= kz - 1) ? waf_half(f1, ex[u], d3, dx[u], xc[u], xb[u]) : T(0);
+          w1 = waf_update(xb[u], dC, h, uC, h1[u], v1, xb[u]);
+          dx[u] = ex[u]; ex[u] = d3; xb[u] = xc[u]; xc[u] = xd; h1[u] = h;
+        }
+        // wz1(t-1) - wz1(t); none at t = 1, and for t > kz wz1 stays at wz1(kz)
+        const T e3 = (FAST || t > 1) ? sub_rn(y3[u], w1) : T(0);
+        y1[u] = y2[u]; y2[u] = y3[u]; y3[u] = w1;
+        if (FAST || m >= 1) {
+          const T h = (FAST || m <= kz - 1) ? waf_half(f2, ey[u], e3, dy[u], y2[u], y1[u]) : T(0);
+          wz[u][c + (unsigned)(m - 1) * pl] = waf_update(y1[u], dA, h, uA, h2[u], v2, y1[u]);
+          h2[u] = h;
+        }
+        dy[u] = ey[u]; ey[u] = e3;
+      }
+      sB = sC; sC = sD;
+      uA = uB; uB = uC; dA = dB; dB = dC;
+    };
+    const int tf = kz - 2 >= 4 ? kz - 2 : 3;  // last step of the fast range
+    for (int t = 1; t <= 3; ++t) step(t, std::false_type());
+    for (int t = 4; t <= tf; ++t) step(t, std::true_type());
+    for (int t = tf + 1; t <= kz + 2; ++t) step(t, std::false_type());
+    return;
+  } else {
   T xa[F], xb[F], xc[F];               // pass-1 window x(t-1), x(t), x(t+1)
   T wfw1[F], wfw2[F];                  // wfw1(t), wfw2(m)
   T y0[F], y1[F], y2[F], y3[F];        // wz1(t-3 .. t)
@@ -1843,6 +1969,7 @@ __device__ __forceinline__ void b_waf_vertical_g(const View<T>& d, const int g, 
   for (int t = 1; t <= 3; ++t) step(t, std::false_type());
   for (int t = 4; t <= tf; ++t) step(t, std::true_type());
   for (int t = tf + 1; t <= kz + 2; ++t) step(t, std::false_type());
+  }
 }
 
 template <class T, int F>
@@ -2027,6 +2154,26 @@ __device__ __forceinline__ void b_waf_horizontal(const View<T>& d, const int bx,
   for (int k = k0; k < k1; ++k) {
     const size_t ko = (size_t)k * pl;
     T mz[2], mfac[2], pn[2], ps_[2], pdv[2], zz[2], zfac[2];
+    Face<T> mf[2], zf[2];
+    T oe = rwe, ow = rww, odv;
+    if constexpr (kFluxForm<T>) {
+      // the faces' velocity terms; the cells' metric terms times the face
+      // velocities (and the squared map factor, non-ROTLLR)
+      for (int n = 0; n < 2; ++n) {
+        const T vm = rot ? rv[n] : mul_rn(rv[n], mrm[n]);
+        mf[n] = face_of(vm > T(0), vm, dtrdy);
+        T cs = mul_rn(rot ? rv[n] : mul_rn(rv[n], prs[n]), rws[n]);
+        T cn = mul_rn(rot ? rvn[n] : mul_rn(rvn[n], prn[n]), rwn[n]);
+        if (!rot) { cs = mul_rn(cs, pmx[n]); cn = mul_rn(cn, pmx[n]); }
+        ps_[n] = cs; pn[n] = cn; pdv[n] = sub_rn(cn, cs);
+        const T um = mul_rn(ru[n], zm[n]);
+        zf[n] = face_of(um > T(0), um, dtrdx);
+      }
+      ow = mul_rn(rot ? ruw : mul_rn(ruw, ormw), ow);
+      oe = mul_rn(rot ? rue : mul_rn(rue, orme), oe);
+      if (!rot) { ow = mul_rn(ow, omx); oe = mul_rn(oe, omx); }
+      odv = sub_rn(oe, ow);
+    } else {
     for (int n = 0; n < 2; ++n) {
       const T vv = rv[n];
       mz[n] = rot ? vv * dtrdy : (vv * mrm[n]) * dtrdy;
@@ -2038,8 +2185,8 @@ __device__ __forceinline__ void b_waf_horizontal(const View<T>& d, const int bx,
       zz[n] = (uu * zm[n]) * dtrdx;
       zfac[n] = rot ? T(0.5) * uu : (T(0.5) * uu) * zm[n];
     }
-    const T oe = rwe, ow = rww;
-    const T odv = rot ? (rue * oe - ruw * ow) : ((rue * orme) * oe - (ruw * ormw) * ow);
+    odv = rot ? (rue * oe - ruw * ow) : ((rue * orme) * oe - (ruw * ormw) * ow);
+    }
     for (int f = 0; f < kNumAdvected; ++f) {
       const T* __restrict__ W = sw[b];
       const T* __restrict__ P = sp[b];
@@ -2052,15 +2199,27 @@ __device__ __forceinline__ void b_waf_horizontal(const View<T>& d, const int bx,
       }
       for (int n = 0; n < 2; ++n) {  // zpby between tile rows r+1 and r+2 (flat: q+HJ, q+2HJ)
         const int q = tid + 256 * n;
-        if (q < NM)
-          smf[q] = mfac[n] * waf_hflux(mz[n], W[q], W[q + HJ], W[q + 2 * HJ], W[q + 3 * HJ]);
+        if (q < NM) {
+          if constexpr (kFluxForm<T>) {
+            const T m2 = W[q], m1 = W[q + HJ], x0 = W[q + 2 * HJ], p1 = W[q + 3 * HJ];
+            const bool pos = mf[n].pos;
+            const T num = sub_rn(pos ? m1 : p1, pos ? m2 : x0);
+            smf[q] = waf_half(mf[n], sub_rn(x0, m1), num, num, m1, x0);
+          } else {
+            smf[q] = mfac[n] * waf_hflux(mz[n], W[q], W[q + HJ], W[q + 2 * HJ], W[q + 3 * HJ]);
+          }
+        }
       }
       __syncthreads();
       for (int n = 0; n < 2; ++n) {  // p0 (:1113-1131, :1222-1240)
         const int q = tid + 256 * n;
         if (q < NP) {
-          const T zdv = pdv[n] * P[q];
           const T wc = W[q + 2 * HJ];
+          if constexpr (kFluxForm<T>) {
+            sp0[q] = waf_update(wc, ps_[n], smf[q], pn[n], smf[q + HJ], pdv[n], P[q]);
+            continue;
+          }
+          const T zdv = pdv[n] * P[q];
           sp0[q] = rot ? ((wc + smf[q] * ps_[n]) - smf[q + HJ] * pn[n]) + zdv
                        : wc + pmx[n] * (((smf[q] * ps_[n]) - smf[q + HJ] * pn[n]) + zdv);
         }
@@ -2070,15 +2229,27 @@ __device__ __forceinline__ void b_waf_horizontal(const View<T>& d, const int bx,
         const int q = tid + 256 * n;
         if (q < NZ) {
           const int z0 = zoff[n];
-          szf[q] = zfac[n] * waf_hflux(zz[n], sp0[z0], sp0[z0 + 1], sp0[z0 + 2], sp0[z0 + 3]);
+          if constexpr (kFluxForm<T>) {
+            const T m2 = sp0[z0], m1 = sp0[z0 + 1], x0 = sp0[z0 + 2], p1 = sp0[z0 + 3];
+            const bool pos = zf[n].pos;
+            const T num = sub_rn(pos ? m1 : p1, pos ? m2 : x0);
+            szf[q] = waf_half(zf[n], sub_rn(x0, m1), num, num, m1, x0);
+          } else {
+            szf[q] = zfac[n] * waf_hflux(zz[n], sp0[z0], sp0[z0 + 1], sp0[z0 + 2], sp0[z0 + 3]);
+          }
         }
       }
       __syncthreads();
       if (ook) {  // new pp (:1173-1187, :1283-1297)
         const T p0 = sp0[op0];
-        const T zdv = odv * P[op0];
-        const T out = rot ? ((p0 + szf[ozf] * ow) - szf[ozf + 1] * oe) + zdv
-                          : p0 + omx * (((szf[ozf] * ow) - szf[ozf + 1] * oe) + zdv);
+        T out;
+        if constexpr (kFluxForm<T>) {
+          out = waf_update(p0, ow, szf[ozf], oe, szf[ozf + 1], odv, P[op0]);
+        } else {
+          const T zdv = odv * P[op0];
+          out = rot ? ((p0 + szf[ozf] * ow) - szf[ozf + 1] * oe) + zdv
+                    : p0 + omx * (((szf[ozf] * ow) - szf[ozf + 1] * oe) + zdv);
+        }
         d.fset[d.fcur ^ 1][f][ko + co] = out;
       }
       if (next_field || next_level) stash(b ^ 1);  // the other buffer was last read two fields ago
@@ -2141,6 +2312,86 @@ __device__ __forceinline__ void b_waf_hstrip(const View<T>& d, const int bx, con
   const bool rot = d.rotllr;
   auto row = [&](int i) { return (size_t)j + (size_t)nj * wrap2(i, ni); };
 
+  if constexpr (kFluxForm<T>) {
+    // Flux form.  Per field: w0, wp1 = wz(i), wz(i+1), da, db =
+    // wz(i)-wz(i-1), wz(i+1)-wz(i), and half the WAF value of the face below
+    // row i; the row's velocity and metric terms are shared by the fields.
+    static_assert(kNumAdvected % G == 0, "fields per group");
+    for (int g0 = 0; g0 < kNumAdvected; g0 += G) {
+      const T* wz[G];
+      const T* pp[G];
+      T* out[G];
+      T w0[G], w1[G], da[G], db[G], vs[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        wz[g] = d.wz + ((size_t)(g0 + g) * kz + k) * pl;
+        pp[g] = d.fset[d.fcur][g0 + g] + (size_t)k * pl;
+        out[g] = d.fset[d.fcur ^ 1][g0 + g] + (size_t)k * pl;
+      }
+      T v_i;  // v at the face below row i (times 1 / msfv, non-ROTLLR)
+      {
+        const size_t r = row(i_s);
+        v_i = rot ? v[r] : mul_rn(v[r], d.rmv[r]);
+        const Face<T> f = face_of(v_i > T(0), v_i, dtrdy);
+        const size_t r2 = row(i_s - 2), r1 = row(i_s - 1), rp = row(i_s + 1);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const T a = wz[g][r2], b = wz[g][r1], cc = wz[g][r], e = wz[g][rp];
+          w0[g] = cc; w1[g] = e;
+          da[g] = sub_rn(cc, b); db[g] = sub_rn(e, cc);
+          vs[g] = waf_half(f, da[g], sub_rn(b, a), db[g], b, cc);
+        }
+      }
+      // the loads of row i+1 are issued while row i is computed
+      T n_wp2[G], n_pold[G];
+      T n_vn, n_rmvn, n_pn, n_ps, n_uu, n_oe, n_ow, n_zm, n_mx2;
+      auto fetch_row = [&](int i) {
+        const size_t r = row(i), rn = row(i + 1), r2 = row(i + 2);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          n_wp2[g] = wz[g][r2];
+          n_pold[g] = pp[g][r];
+        }
+        n_vn = v[rn];
+        n_rmvn = rot ? T(1) : d.rmv[rn];
+        n_pn = wn_[r]; n_ps = ws_[r];
+        n_uu = u[r];
+        n_oe = we_[r]; n_ow = ww_[r];
+        n_zm = rot ? d.mu[r] : d.rmu[r];
+        n_mx2 = rot ? T(1) : d.mx2[r];
+      };
+      fetch_row(i_s);
+      for (int i = i_s; i < i_e; ++i) {
+        const size_t r = row(i);
+        const T v_n = rot ? n_vn : mul_rn(n_vn, n_rmvn);
+        const T um = mul_rn(n_uu, n_zm), uf = rot ? n_uu : um;
+        const T ufe = __shfl_down_sync(0xffffffffu, uf, 1);  // u(j+1)
+        T cs = mul_rn(v_i, n_ps), cn = mul_rn(v_n, n_pn), cw = mul_rn(uf, n_ow), ce = mul_rn(ufe, n_oe);
+        if (!rot) { cs = mul_rn(cs, n_mx2); cn = mul_rn(cn, n_mx2); cw = mul_rn(cw, n_mx2); ce = mul_rn(ce, n_mx2); }
+        const T pdv = sub_rn(cn, cs), odv = sub_rn(ce, cw);
+        const Face<T> fm = face_of(v_n > T(0), v_n, dtrdy), fz = face_of(um > T(0), um, dtrdx);
+        T wp2v[G], poldv[G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) { wp2v[g] = n_wp2[g]; poldv[g] = n_pold[g]; }
+        if (i + 1 < i_e) fetch_row(i + 1);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const T dn = sub_rn(wp2v[g], w1[g]);
+          const T vn = waf_half(fm, db[g], da[g], dn, w0[g], w1[g]);  // face between rows i and i+1
+          const T p0 = waf_update(w0[g], cs, vs[g], cn, vn, pdv, poldv[g]);
+          w0[g] = w1[g]; w1[g] = wp2v[g]; da[g] = db[g]; db[g] = dn; vs[g] = vn;
+          const T pm1 = __shfl_up_sync(0xffffffffu, p0, 1);
+          const T dz = sub_rn(p0, pm1);  // across the face between j-1 and j
+          const T dzm = __shfl_up_sync(0xffffffffu, dz, 1), dzp = __shfl_down_sync(0xffffffffu, dz, 1);
+          const T vw = waf_half(fz, dz, dzm, dzp, pm1, p0);
+          const T ve = __shfl_down_sync(0xffffffffu, vw, 1);  // face between j and j+1
+          if (out_lane) out[g][r] = waf_update(p0, cw, vw, ce, ve, odv, poldv[g]);
+        }
+        v_i = v_n;
+      }
+    }
+    return;
+  } else {
   for (int g0 = 0; g0 < kNumAdvected; g0 += G) {
     const int ng = min(G, kNumAdvected - g0);
     const T* wz[G];
@@ -2234,6 +2485,7 @@ __device__ __forceinline__ void b_waf_hstrip(const View<T>& d, const int bx, con
       }
       v_i = v_n; rmv_i = rmv_n;
     }
+  }
   }
 }
 
