@@ -281,6 +281,9 @@ size_t layout(View<T>& v, char* base, const moloch_handle* h) {
   v.eu_j = T1(ne); v.eu_i = T1(ne); v.ev_j = T1(ne); v.ev_i = T1(ne); v.ep_j = T1(ne); v.ep_i = T1(ne);
   v.fmz = T3(); v.fmzf = T3p(); v.zeta = T3(); v.dz = T3();
   v.rfw = T3(); v.rfs = T3();
+  v.fmx = v.fzd = nullptr;
+  v.mo1 = v.mo2 = nullptr;
+  if (h->prm.mode == MOLOCH_FP64) { v.fmx = T3(); v.fzd = T3(); v.mo1 = T3(); v.mo2 = T3(); }
   v.wafu = T3(); v.wafd = T3(); v.wafn = T3(); v.wafs = T3(); v.wafe = T3(); v.wafw = T3();
   v.hx = T2(); v.hy = T2(); v.mx = T2(); v.mu = T2(); v.mv = T2(); v.rmu = T2(); v.rmv = T2();
   v.mx2 = T2(); v.coru = T2(); v.corv = T2();
@@ -618,6 +621,8 @@ int init_impl(moloch_handle* h, View<T>& v) {
   // 3-D static terms
   const size_t n3 = pl * kz;
   std::vector<double> rfw(n3), rfs(n3), wu(n3), wd(n3), wn(n3), ws(n3), we(n3), ww(n3), dz(n3);
+  const bool lean = P.mode == MOLOCH_FP64;
+  std::vector<double> fmx(lean ? n3 : 0), fzd(lean ? n3 : 0);
   host_parallel((size_t)kz * ni, [&](size_t r0, size_t r1) {
     for (size_t r = r0; r < r1; ++r) {
       const int k = (int)(r / ni) + 1, i = (int)(r % ni) + 1;
@@ -646,6 +651,13 @@ int init_impl(moloch_handle* h, View<T>& v) {
           ww[q] = ((dtrdx_a * 2.0) * f) / (f + fw);
         }
         dz[q] = dzita / f;  // layer thickness for the column sums
+        if (lean) {
+          const double mxx2 = mxx * mxx;
+          rfw[q] = P.rotllr ? dtrdx * rfw[q] : (dtrdx * rfw[q]) / muu;
+          rfs[q] = (dtrdy * rfs[q]) * rmvs;
+          fmx[q] = f * (P.rotllr ? mxx : mxx2);
+          fzd[q] = f * dtrdz;
+        }
       }
     }
   });
@@ -656,6 +668,7 @@ int init_impl(moloch_handle* h, View<T>& v) {
   if ((rc = up3(v.wafn, wn)) || (rc = up3(v.wafs, ws)) || (rc = up3(v.wafe, we)) || (rc = up3(v.wafw, ww)))
     return rc;
   if ((rc = up3(v.dz, dz))) return rc;
+  if (lean && ((rc = up3(v.fmx, fmx)) || (rc = up3(v.fzd, fzd)))) return rc;
   // w(:,:,1) = 0 (:260-262); s, deltaw zero (reset_tendencies :1313-1325 --
   // the kernels never write s(1), deltaw(1), deltaw(kz+1), which therefore
   // keep this zero for the whole run)
@@ -1403,7 +1416,7 @@ int moloch_gpu_autotune(moloch_handle_t* h, int* choice, double* best_ms, int n)
     if ((cand & 512) && !(cand & 16)) continue;  // levels per warp of the fused strips
     if ((cand & 64) && (h->elem != 4 || !(cand & 8) || h->nj() % 2)) continue;  // two-column strips: FP32, jx even
     if ((cand & 12) == 12) continue;  // strips replace the k-marching momentum
-    if ((cand & 16) && (cand & 3)) continue;  // the fused kernel replaces both
+    if ((cand & 16) && ((cand & 3) || h->prm.mode == MOLOCH_FP64)) continue;  // the fused kernel replaces both
     if ((cand & 32) && !staged_ok) continue;  // staged column solve: FP32 domains with tensor maps
     h->vd.kmarch = cand;
     h->vf.kmarch = cand;
@@ -1863,7 +1876,7 @@ int moloch_gpu_ensemble_autotune(moloch_ensemble_t* e, int* choice, double* best
   for (int c2 = 0; c2 < 128; ++c2) {
     const int cand = (c2 & 63) | ((c2 & 64) ? 512 : 0);
     if ((cand & 12) == 12) continue;  // strips replace the k-marching momentum
-    if ((cand & 16) && (cand & 3)) continue;  // the fused kernel replaces both
+    if ((cand & 16) && ((cand & 3) || e->elem == 8)) continue;  // the fused kernel replaces both
     if ((cand & 32) && !staged_ok) continue;  // batched staged column solve: FP32 members with tensor maps
     if ((cand & 512) && !(cand & 16)) continue;  // two levels per warp of the fused strips
     e->kmarch = cand;

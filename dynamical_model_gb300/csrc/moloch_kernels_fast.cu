@@ -1,7 +1,6 @@
 // FP64 and FP32-storage kernels with multiply-add contraction allowed.
 #define MOLOCH_KNS kfast
-#define MOLOCH_NR_DDIV 1       // qdiv of FP64 by Newton-Raphson (div_nr)
-#define MOLOCH_FLUX_LIMITER 1  // WAF limiter in flux form
+#define MOLOCH_LEAN_FP64 1  // FP64 expressions written for few FP64 operations
 #include "../../include/moloch_gb300.h"
 #include "moloch_kernels.cuh"
 

@@ -25,8 +25,7 @@
 // its next barrier, and a launch that starts with *err set returns at once,
 // so a failed step never waits longer than one limit per block.
 #define MOLOCH_KNS kpersist
-#define MOLOCH_NR_DDIV 1       // qdiv of FP64 by Newton-Raphson (div_nr)
-#define MOLOCH_FLUX_LIMITER 1  // WAF limiter in flux form
+#define MOLOCH_LEAN_FP64 1  // FP64 expressions written for few FP64 operations
 #include "../../include/moloch_gb300.h"
 #include "moloch_kernels.cuh"
 #include "moloch_persist.h"

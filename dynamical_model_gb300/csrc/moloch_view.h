@@ -50,6 +50,8 @@ struct View {
   T* deltaw;  // kz+1 levels
   T* zdiv2a;  // horizontal divergence (Equation 16)
   T* zdiv2b;  // after divdamp and the vertical s term
+  T* mo1;  // moist factors of the Exner/theta update, written by a sound()
+  T* mo2;  // call's first substep and read by the others (kLean)
   double* wp;    // Thomas down-sweep values (FP64 in every mode), kz+1 levels
   double* wwkw;  // Thomas pivot ratios (FP64 in every mode), kz+1 levels
   T* ux;
@@ -76,8 +78,14 @@ struct View {
   const T* fmzf;  // kz+1 levels
   const T* zeta;
   const T* dz;
-  const T* rfw;   // 2 / (fmz(j) + fmz(j-1))
-  const T* rfs;   // 2 / (fmz(i) + fmz(i-1))
+  // rfw, rfs: 2 / (fmz(j) + fmz(j-1)), 2 / (fmz(i) + fmz(i-1)).  MOLOCH_FP64
+  // (the contracting FP64 build, kLean) holds every static factor of
+  // Equation 16 in them, dtrdx (rmu) rfw and dtrdy rmv rfs, and has three
+  // more arrays (nullptr elsewhere)
+  const T* rfw;
+  const T* rfs;
+  const T* fmx;   // fmz mx (ROTLLR) or fmz mx2
+  const T* fzd;   // fmz dtrdz
   const T* wafu;  // wafone zrfmu
   const T* wafd;  // wafone zrfmd
   const T* wafn;  // wafone zrfmn

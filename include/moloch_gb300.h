@@ -213,9 +213,9 @@ int moloch_gpu_set_wait_limit(moloch_handle_t* h, long long cycles, int skip_job
 int moloch_gpu_check_division(const float* a, const float* b, float* q_corr, float* q_ieee, int n, void* stream);
 
 /* The same for FP64 (tests): q_nr = the quotient the contracting build's
- * WAF limiter uses (FP32 reciprocal estimate, two Newton-Raphson steps, one
- * residual correction) and q_ieee = CUDA's IEEE FP64 quotient.  No
- * reference counterpart. */
+ * diagnostics and column solve use (FP32 reciprocal estimate, two residual
+ * corrections) and q_ieee = CUDA's IEEE FP64 quotient.  No reference
+ * counterpart. */
 int moloch_gpu_check_division_f64(const double* a, const double* b, double* q_nr, double* q_ieee, int n,
                                   void* stream);
 
@@ -251,7 +251,7 @@ const char* moloch_gpu_kernel_name(int kind);
  *               thread, next level prefetched), 8 momentum as warp strips
  *               (30 columns x 32 rows), 16 divergence and damping fused in
  *               one warp-strip kernel (29 columns x 32 rows; overrides 1
- *               and 2), 32 the implicit-w column solve staged by TMA with
+ *               and 2; MOLOCH_FP64 ignores it), 32 the implicit-w column solve staged by TMA with
  *               its column state in TMEM (FP32 storage, jx a multiple of 4,
  *               kz <= 64; elsewhere the bit is ignored), 64 (with 8) the
  *               momentum strips with two columns per lane (62 columns x 32
