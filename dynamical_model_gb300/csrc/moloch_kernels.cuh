@@ -1618,6 +1618,104 @@ __global__ void __launch_bounds__(128, 5) k_momentum_strip2(View<float> d, int R
   b_momentum_strip2(d, blockIdx.x, blockIdx.y, R, ring[threadIdx.x >> 5], threadIdx.x >> 5, 4);
 }
 
+// ---- momentum with four columns per thread (FP32, jx a multiple of 4) -----
+// One thread per quad of columns, row and level: every array of the stencil
+// is read with 16-byte loads, all issued before the first use, the west and
+// east neighbours come from the lanes beside (from memory on the warp's end
+// lanes), and the stale-halo rows of the reference (:716-735) are read
+// through the row pointers, so no column tests them.
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+constexpr int kQuadY = 4;  // rows of a block of the quad kernels, one warp (128 columns) each
+
+__global__ void __launch_bounds__(32 * kQuadY, 5) k_momentum_quad(const __grid_constant__ View<float> d) {
+  if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
+  const int nj = d.nj, ni = d.ni, k = blockIdx.z;
+  const unsigned pl = (unsigned)d.pl, o = (unsigned)k * pl;
+  const int lane = threadIdx.x, ii = blockIdx.y * kQuadY + threadIdx.y;
+  if (ii >= ni) return;  // whole warp
+  const int jq = 4 * (blockIdx.x * 32 + lane);
+  const bool in = jq < nj;
+  const int j0 = in ? jq : 0;  // lanes past the row repeat its first quad
+  const unsigned r = (unsigned)nj * ii, rs = (unsigned)nj * wm1(ii, ni), ej = (unsigned)ni * k, ei = (unsigned)nj * k;
+  const float* __restrict__ u = d.ubuf[d.cur] + o + r;
+  const float* __restrict__ v = d.vbuf[d.cur] + o + r;
+  const float* __restrict__ t = d.tetav + o;
+  const float* __restrict__ p = d.pai + o + r;
+  const float* __restrict__ dw = d.deltaw + o;
+  // rows i-1 and i+1 whose periodic image is the older halo value
+  const float* __restrict__ us = ii == 0 ? d.eu_i + ei : u - nj;
+  const float* __restrict__ ps = ii == 0 ? d.ep_i + ei : p - nj;
+  const float* __restrict__ vn = ii == ni - 1 ? d.ev_i + ei : v + nj;
+  const float4 U = ld4(u + j0), V = ld4(v + j0), T = ld4(t + r + j0), P = ld4(p + j0);
+  const float4 D0 = ld4(dw + r + j0), D1 = ld4(dw + pl + r + j0);
+  const float4 US = ld4(us + j0), VN = ld4(vn + j0), TS = ld4(t + rs + j0), PS = ld4(ps + j0);
+  const float4 S0 = ld4(dw + rs + j0), S1 = ld4(dw + pl + rs + j0);
+  const float4 CU = ld4(d.coru + r + j0), CV = ld4(d.corv + r + j0), HX = ld4(d.hx + r + j0), HY = ld4(d.hy + r + j0);
+  const float4 MU = ld4(d.mu + r + j0);
+  const bool rot = d.rotllr;
+  const float4 MV = rot ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4(d.mv + r + j0);
+  // column j0-1 of v, v(i+1), tetav, pai, deltaw and column j0+4 of u, u(i-1)
+  float vw = 0.f, vnw = 0.f, tw = 0.f, pw = 0.f, dw0 = 0.f, dw1 = 0.f, ue = 0.f, use = 0.f;
+  if (lane == 0) {
+    if (j0 == 0) {
+      vw = d.ev_j[ej + ii]; vnw = d.ev_j[ej + wp1(ii, ni)]; pw = d.ep_j[ej + ii];
+    } else {
+      vw = v[j0 - 1]; vnw = vn[j0 - 1]; pw = p[j0 - 1];
+    }
+    const unsigned jw = r + (j0 == 0 ? nj : j0) - 1;
+    tw = t[jw]; dw0 = dw[jw]; dw1 = dw[pl + jw];
+  }
+  if (lane == 31 || j0 + 4 >= nj) {
+    if (j0 + 4 >= nj) {
+      ue = d.eu_j[ej + ii]; use = d.eu_j[ej + wm1(ii, ni)];
+    } else {
+      ue = u[j0 + 4]; use = us[j0 + 4];
+    }
+  }
+  auto west = [&](float x, float own) {
+    const float y = __shfl_up_sync(0xffffffffu, x, 1);
+    return lane == 0 ? own : y;
+  };
+  auto east = [&](float x, float own) {
+    const float y = __shfl_down_sync(0xffffffffu, x, 1);
+    return lane == 31 || j0 + 4 >= nj ? own : y;
+  };
+  vw = west(V.w, vw); vnw = west(VN.w, vnw); tw = west(T.w, tw); pw = west(P.w, pw);
+  dw0 = west(D0.w, dw0); dw1 = west(D1.w, dw1);
+  ue = east(U.x, ue); use = east(US.x, use);
+  const float dts = d.dts, egdts = d.egdts, dtrdx = d.dtrdx, dtrdy = d.dtrdy, hcpd = 0.5f * float(kCpd);
+  const float gzh = d.gzitakh[k];
+  auto eq17 = [&](float cu, float cv, float wv, float wvn, float cvn, float wt, float ct, float wp, float cp, float wd0,
+                  float wd1, float cd0, float cd1, float coru, float hx, float mu) {
+    const float zcx = dtrdx * mu;
+    const float zfz = egdts + 0.25f * (((wd0 + wd1) + cd0) + cd1);
+    const float zrom1u = hcpd * (wt + ct);
+    const float zcor1u = ((coru * dts) * 0.25f) * (((cv + wv) + wvn) + cvn);
+    return ((cu + zcor1u) - (zfz * hx) * gzh) - (zcx * zrom1u) * (cp - wp);
+  };
+  auto eq18 = [&](float cv, float cu, float su, float eu, float esu, float st, float ct, float sp, float cp, float sd0,
+                  float sd1, float cd0, float cd1, float corv, float hy, float mv) {
+    const float zcy = rot ? dtrdy : dtrdy * mv;
+    const float zfz = egdts + 0.25f * (((sd0 + sd1) + cd0) + cd1);
+    const float zrom1v = hcpd * (st + ct);
+    const float zcor1v = ((corv * dts) * 0.25f) * (((cu + su) + eu) + esu);
+    return ((cv - zcor1v) - (zfz * hy) * gzh) - (zcy * zrom1v) * (cp - sp);
+  };
+  if (!in) return;
+  const unsigned c = o + r + j0;
+  st4(d.ubuf[d.cur ^ 1] + c,
+      make_float4(eq17(U.x, V.x, vw, vnw, VN.x, tw, T.x, pw, P.x, dw0, dw1, D0.x, D1.x, CU.x, HX.x, MU.x),
+                  eq17(U.y, V.y, V.x, VN.x, VN.y, T.x, T.y, P.x, P.y, D0.x, D1.x, D0.y, D1.y, CU.y, HX.y, MU.y),
+                  eq17(U.z, V.z, V.y, VN.y, VN.z, T.y, T.z, P.y, P.z, D0.y, D1.y, D0.z, D1.z, CU.z, HX.z, MU.z),
+                  eq17(U.w, V.w, V.z, VN.z, VN.w, T.z, T.w, P.z, P.w, D0.z, D1.z, D0.w, D1.w, CU.w, HX.w, MU.w)));
+  st4(d.vbuf[d.cur ^ 1] + c,
+      make_float4(eq18(V.x, U.x, US.x, U.y, US.y, TS.x, T.x, PS.x, P.x, S0.x, S1.x, D0.x, D1.x, CV.x, HY.x, MV.x),
+                  eq18(V.y, U.y, US.y, U.z, US.z, TS.y, T.y, PS.y, P.y, S0.y, S1.y, D0.y, D1.y, CV.y, HY.y, MV.y),
+                  eq18(V.z, U.z, US.z, U.w, US.w, TS.z, T.z, PS.z, P.z, S0.z, S1.z, D0.z, D1.z, CV.z, HY.z, MV.z),
+                  eq18(V.w, U.w, US.w, ue, use, TS.w, T.w, PS.w, P.w, S0.w, S1.w, D0.w, D1.w, CV.w, HY.w, MV.w)));
+}
+
 // ---- divergence + divdamp as warp strips (:514-597, :853-895, :627-630) ---
 // The work of k_sound_div and k_sound_damp in one pass.  One warp per strip
 // of kDDJ output columns x R rows of one level k, lanes on columns
@@ -3122,7 +3220,11 @@ int launch_sound(View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
     }
     bool pairs = false;
     if constexpr (sizeof(T) == 4) {
-      if ((d.kmarch & 8) && (d.kmarch & 64) && d.nj % 2 == 0) {  // two columns per lane
+      if ((d.kmarch & 8) && (d.kmarch & 64) && d.nj % 4 == 0) {  // four columns per thread
+        const dim3 g4((d.nj / 4 + 31) / 32, (d.ni + kQuadY - 1) / kQuadY, d.kz);
+        MOLOCH_LAUNCH(KK_SOUND_MOMENTUM, st, k_momentum_quad<<<g4, dim3(32, kQuadY), 0, st>>>(d));
+        pairs = true;
+      } else if ((d.kmarch & 8) && (d.kmarch & 64) && d.nj % 2 == 0) {  // two columns per lane
         const int nstrips = ((d.nj + 1 + kMom2J - 1) / kMom2J) * ((d.ni + d.srows - 1) / d.srows);
         MOLOCH_LAUNCH(KK_SOUND_MOMENTUM, st,
                       k_momentum_strip2<<<dim3((nstrips + 3) / 4, d.kz), 128, 0, st>>>(d, d.srows));
