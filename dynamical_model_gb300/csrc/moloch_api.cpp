@@ -228,7 +228,7 @@ struct moloch_handle {
   moloch::mlp::Surrogate* sur = nullptr;
   // TMA tensor maps of the staged column kernel (FP32 storage), one set per
   // advected-field buffer set
-  alignas(64) unsigned char cmaps[10240];
+  alignas(64) unsigned char cmaps[4096];
   int nj() const { return grid.jx; }
   int ni() const { return grid.iy; }
   int kz() const { return grid.kz; }
@@ -302,6 +302,7 @@ size_t layout(View<T>& v, char* base, const moloch_handle* h) {
   v.stag4 = 0;
   v.sur_skip = nullptr;
   v.cmaps = nullptr;
+  v.twide = 1;
   v.spin_cycles = kDefaultSpinCycles;
   v.fault_skip_job = -1;
   return off + 256;
@@ -678,6 +679,7 @@ int init_impl(moloch_handle* h, View<T>& v) {
   CUDA_TRY(cudaStreamSynchronize(h->stream));
   if constexpr (sizeof(T) == sizeof(float)) {
     v.cmaps = nullptr;
+    v.twide = kfast::column_wide(nj, ni);
     if (kfast::column_maps_bytes() <= (int)sizeof(h->cmaps) && kfast::build_column_maps(v, h->cmaps))
       v.cmaps = h->cmaps;
   }
@@ -1412,7 +1414,7 @@ int moloch_gpu_autotune(moloch_handle_t* h, int* choice, double* best_ms, int n)
   int pick1 = h->elem == 8 ? h->vd.kmarch : h->vf.kmarch;
   const bool staged_ok = h->elem == 4 && h->vf.cmaps != nullptr;
   for (int cand = 0; cand < 1024; ++cand) {
-    if ((cand & 384) && (!(cand & 32) || (cand & 384) == 384)) continue;  // one staged-column variant
+    if (!(cand & 32) != !(cand & 128) || (cand & 256)) continue;  // the staged column solve (128, 256: the same kernel)
     if ((cand & 512) && !(cand & 16)) continue;  // levels per warp of the fused strips
     if ((cand & 64) && (h->elem != 4 || !(cand & 8) || h->nj() % 2)) continue;  // two-column strips: FP32, jx even
     if ((cand & 12) == 12) continue;  // strips replace the k-marching momentum
@@ -1584,8 +1586,9 @@ void ens_tiles(moloch_ensemble* e) {
     for (int y = 0; y < (ni + 3) / 4; ++y)
       for (int x = 0; x < tj; ++x) e->tiles[TK_COLUMN].push_back(make_int4(q, x, y, 0));
     if (e->elem == 4 && e->m[q]->vf.cmaps) {
-      for (int y = 0; y < (ni + kTwRows - 1) / kTwRows; ++y)
-        for (int x = 0; x < tj; ++x) e->tiles[TK_COLTW].push_back(make_int4(q, x, y, 0));
+      const int wide = e->m[q]->vf.twide;
+      for (int y = 0; y < (ni * wide + kTwWarps - 1) / kTwWarps; ++y)
+        for (int x = 0; x < (tj + wide - 1) / wide; ++x) e->tiles[TK_COLTW].push_back(make_int4(q, x, y, 0));
     } else {
       for (int y = 0; y < (ni + 3) / 4; ++y)
         for (int x = 0; x < tj; ++x) e->tiles[TK_COLREST].push_back(make_int4(q, x, y, 0));
@@ -1681,12 +1684,12 @@ int ens_upload(moloch_ensemble* e, Batch<T>& b, View<T> moloch_handle::*vm) {
     off += (e->tiles[t].size() * sizeof(int4) + 255) & ~size_t(255);
   }
   b.cmaps = nullptr;
-  if (staged) {  // the 12-row boxes (map config 1) of each member, both parities
+  if (staged) {  // the maps of each member, both parities
     std::vector<unsigned char> hm(cm_bytes, 0);
     for (int q = 0; q < n; ++q)
       if (e->m[q]->vf.cmaps)
         std::memcpy(hm.data() + 2 * set_bytes * q,
-                    static_cast<const unsigned char*>(e->m[q]->vf.cmaps) + 2 * set_bytes, 2 * set_bytes);
+                    static_cast<const unsigned char*>(e->m[q]->vf.cmaps), 2 * set_bytes);
     CUDA_TRY(cudaMemcpy(p + off, hm.data(), cm_bytes, cudaMemcpyHostToDevice));
     b.cmaps = p + off;
     off += (cm_bytes + 255) & ~size_t(255);

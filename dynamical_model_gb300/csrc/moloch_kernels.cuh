@@ -85,7 +85,7 @@ __device__ __forceinline__ int wp2(int x, int n) { int y = x + 2; return y >= n 
 // a*b - c*d and a*b + c*d with the multiply-add contraction fixed in FP32
 // storage: left to the compiler either product may be fused, and which one
 // it fuses depends on the code around the expression, so the same body in
-// two kernels (k_sound_column and k_sound_column_tm; a batched kernel and
+// two kernels (k_sound_column and k_sound_column_tw; a batched kernel and
 // the persistent ensemble kernel) could round differently.  FP64 keeps the
 // expression as written (the exact build contracts nothing).
 __device__ __forceinline__ float prod_sub(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
@@ -3127,8 +3127,7 @@ template <class T>
 inline bool column_tm_ok(const View<T>& d) {
   return sizeof(T) == 4 && (d.kmarch & 32) && d.cmaps != nullptr;
 }
-// persistent column kernels: one CTA per SM, at most one per tile
-inline int persistent_grid(int ntiles) {
+inline int sm_count() {
   static int nsm = 0;
   if (!nsm) {
     int dev = 0;
@@ -3136,11 +3135,18 @@ inline int persistent_grid(int ntiles) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (nsm <= 0) nsm = 1;
   }
-  return ntiles < nsm ? ntiles : nsm;
+  return nsm;
 }
-inline int column_tm_grid(int nj, int ni) { return persistent_grid(((nj + 31) / 32) * ((ni + 3) / 4)); }
+// persistent CTAs of the staged column solve over ntiles tiles
+inline int column_tw_grid(int ntiles) {
+  const int slots = TwCfg<0>::ctas * sm_count();
+  return ntiles < slots ? ntiles : slots;
+}
 template <class T>
-inline int column_tm_grid(const View<T>& d) { return column_tm_grid(d.nj, d.ni); }
+inline int column_tw_grid(const View<T>& d) {
+  const int w = d.twide;
+  return column_tw_grid(((d.nj + 32 * w - 1) / (32 * w)) * ((d.ni * w + kTwWarps - 1) / kTwWarps));
+}
 
 // one sound() call: nsound substeps; flips d.cur once per substep, twice
 // with the fused divergence/damping kernel (kmarch bit 16)
@@ -3189,29 +3195,14 @@ int launch_sound(View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
       bool staged = false;
       if constexpr (sizeof(T) == 4) {
         if (column_tm_ok(d)) {
-          // bits 128 / 256: two words of column state a level, 12 / 16 rows
-          const int cfg = (d.kmarch & 256) ? 2 : (d.kmarch & 128) ? 1 : 0;
-          const ColumnMaps& cm = static_cast<const ColumnMaps*>(d.cmaps)[2 * cfg + d.fcur];
-          const int grid = column_tm_grid(d);
-          if (cfg == 2) {
-            if (last)
-              MOLOCH_LAUNCH(KK_SOUND_COLUMN_TM, st,
-                            k_sound_column_tw<T, 1, 16><<<grid, TwCfg<16>::threads, TwCfg<16>::smem, st>>>(d, cm, ns));
-            else
-              MOLOCH_LAUNCH(KK_SOUND_COLUMN_TM, st,
-                            k_sound_column_tw<T, 0, 16><<<grid, TwCfg<16>::threads, TwCfg<16>::smem, st>>>(d, cm, ns));
-          } else if (cfg == 1) {
-            if (last)
-              MOLOCH_LAUNCH(KK_SOUND_COLUMN_TM, st,
-                            k_sound_column_tw<T, 1, 12><<<grid, TwCfg<12>::threads, TwCfg<12>::smem, st>>>(d, cm, ns));
-            else
-              MOLOCH_LAUNCH(KK_SOUND_COLUMN_TM, st,
-                            k_sound_column_tw<T, 0, 12><<<grid, TwCfg<12>::threads, TwCfg<12>::smem, st>>>(d, cm, ns));
-          } else if (last) {
-            MOLOCH_LAUNCH(KK_SOUND_COLUMN_TM, st, k_sound_column_tm<T, 1><<<grid, kTmThreads, kTmSmem, st>>>(d, cm, ns));
-          } else {
-            MOLOCH_LAUNCH(KK_SOUND_COLUMN_TM, st, k_sound_column_tm<T, 0><<<grid, kTmThreads, kTmSmem, st>>>(d, cm, ns));
-          }
+          const ColumnMaps& cm = static_cast<const ColumnMaps*>(d.cmaps)[d.fcur];
+          const int grid = column_tw_grid(d);
+          if (last)
+            MOLOCH_LAUNCH(KK_SOUND_COLUMN_TM, st,
+                          k_sound_column_tw<T, 1><<<grid, TwCfg<1>::threads, TwCfg<1>::smem, st>>>(d, cm, ns));
+          else
+            MOLOCH_LAUNCH(KK_SOUND_COLUMN_TM, st,
+                          k_sound_column_tw<T, 0><<<grid, TwCfg<0>::threads, TwCfg<0>::smem, st>>>(d, cm, ns));
           staged = true;
         }
       }
@@ -3381,18 +3372,17 @@ int blaunch_step(const Batch<T>& b, cudaStream_t st, const PhaseFlags& fl, int& 
           if ((b.kmarch & 32) && b.cmaps) {
             // the staged column solve over the tiles of the members with
             // tensor maps, the one-thread kernel over the others
-            using TC = TwCfg<kTwRows>;
             const int ntw = b.ntiles[TK_COLTW], nrest = b.ntiles[TK_COLREST];
             const ColumnMaps* cms = static_cast<const ColumnMaps*>(b.cmaps);
             if (ntw > 0) {
-              const int grid = persistent_grid(ntw);
+              const int grid = column_tw_grid(ntw);
               if (last)
                 MOLOCH_LAUNCH(KK_SOUND_COLUMN, st,
-                              kb_sound_column_tw<T, 1, kTwRows><<<grid, TC::threads, TC::smem, st>>>(
+                              kb_sound_column_tw<T, 1><<<grid, TwCfg<1>::threads, TwCfg<1>::smem, st>>>(
                                   V(), cms, b.tiles[TK_COLTW], ntw, fcur, ns, b.kerr, b.spin));
               else
                 MOLOCH_LAUNCH(KK_SOUND_COLUMN, st,
-                              kb_sound_column_tw<T, 0, kTwRows><<<grid, TC::threads, TC::smem, st>>>(
+                              kb_sound_column_tw<T, 0><<<grid, TwCfg<0>::threads, TwCfg<0>::smem, st>>>(
                                   V(), cms, b.tiles[TK_COLTW], ntw, fcur, ns, b.kerr, b.spin));
             }
             if (nrest > 0) {

@@ -45,11 +45,11 @@ EncodeTiledFn encode_tiled() {
   });
   return fn;
 }
-// dense FP32 field (nj, ni, nk), j fastest, as boxes of 32 x rows x levels
-bool map3(EncodeTiledFn fn, CUtensorMap* m, const float* base, int nj, int ni, int nk, int rows, int levels) {
+// dense FP32 field (nj, ni, nk), j fastest, as boxes of cols x rows x levels
+bool map3(EncodeTiledFn fn, CUtensorMap* m, const float* base, int nj, int ni, int nk, int cols, int rows, int levels) {
   const cuuint64_t dims[3] = {(cuuint64_t)nj, (cuuint64_t)ni, (cuuint64_t)nk};
   const cuuint64_t strides[2] = {(cuuint64_t)nj * 4, (cuuint64_t)nj * ni * 4};
-  const cuuint32_t box[3] = {32, (cuuint32_t)rows, (cuuint32_t)levels};
+  const cuuint32_t box[3] = {(cuuint32_t)cols, (cuuint32_t)rows, (cuuint32_t)levels};
   const cuuint32_t es[3] = {1, 1, 1};
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, es,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -57,52 +57,46 @@ bool map3(EncodeTiledFn fn, CUtensorMap* m, const float* base, int nj, int ni, i
 }
 }  // namespace
 
-int column_maps_bytes() { return (int)(2 * kColumnMapConfigs * sizeof(ColumnMaps)); }
+int column_maps_bytes() { return (int)(2 * sizeof(ColumnMaps)); }
 int column_map_set_bytes() { return (int)sizeof(ColumnMaps); }
 
-// the box shapes of the staged column kernels, in the order of the configs
-// (ColumnMaps sets 2 cfg + buffer-set parity)
-static const int kMapRows[kColumnMapConfigs] = {kTmRows, 12, 16};
-static const int kMapLevels[kColumnMapConfigs] = {kKCT, TwCfg<12>::kct, TwCfg<16>::kct};
+// Warps of a column tile side by side along j (8, 4, 2 or 1): the shape that
+// covers the domain with the fewest tiles, the widest of equals (longer runs
+// of DRAM: moloch_column_tm.cuh)
+int column_wide(int nj, int ni) {
+  int best = 1;
+  long tiles = 0;
+  for (int w = kTwWarps; w >= 1; w /= 2) {
+    const long n = (long)((nj + 32 * w - 1) / (32 * w)) * ((ni * w + kTwWarps - 1) / kTwWarps);
+    if (!tiles || n < tiles) { tiles = n; best = w; }
+  }
+  return best;
+}
 
 bool build_column_maps(const View<float>& v, void* out) {
-  if (v.kz > kTmMaxKz || v.kz < 2 || v.nj % 4 != 0 || ((uintptr_t)out & 63)) return false;
+  if (v.kz > kTwMaxKz || v.kz < 2 || v.nj % 4 != 0 || ((uintptr_t)out & 63)) return false;
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return false;
   static std::once_flag attr;
   std::call_once(attr, [] {
-    cudaFuncSetAttribute(k_sound_column_tm<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTmSmem);
-    cudaFuncSetAttribute(k_sound_column_tm<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTmSmem);
-    cudaFuncSetAttribute(k_sound_column_tw<float, 0, 12>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         TwCfg<12>::smem);
-    cudaFuncSetAttribute(k_sound_column_tw<float, 1, 12>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         TwCfg<12>::smem);
-    cudaFuncSetAttribute(k_sound_column_tw<float, 0, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         TwCfg<16>::smem);
-    cudaFuncSetAttribute(k_sound_column_tw<float, 1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         TwCfg<16>::smem);
-    cudaFuncSetAttribute(kb_sound_column_tw<float, 0, kTwRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         TwCfg<kTwRows>::smem);
-    cudaFuncSetAttribute(kb_sound_column_tw<float, 1, kTwRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         TwCfg<kTwRows>::smem);
+    cudaFuncSetAttribute(k_sound_column_tw<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<0>::smem);
+    cudaFuncSetAttribute(k_sound_column_tw<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<1>::smem);
+    cudaFuncSetAttribute(kb_sound_column_tw<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<0>::smem);
+    cudaFuncSetAttribute(kb_sound_column_tw<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<1>::smem);
   });
   ColumnMaps* cm = static_cast<ColumnMaps*>(out);
   const int nj = v.nj, ni = v.ni, kz = v.kz;
-  for (int cfg = 0; cfg < kColumnMapConfigs; ++cfg) {
-    const int r = kMapRows[cfg], l = kMapLevels[cfg];
-    for (int set = 0; set < 2; ++set) {
-      CUtensorMap* m = cm[2 * cfg + set].m;
-      const bool ok =
-          map3(fn, &m[CM_W], v.w, nj, ni, kz + 1, r, l) && map3(fn, &m[CM_FMZF], v.fmzf, nj, ni, kz + 1, r, l) &&
-          map3(fn, &m[CM_QV], v.fset[set][5], nj, ni, kz, r, l) &&
-          map3(fn, &m[CM_TET], v.fset[set][0], nj, ni, kz, r, l) &&
-          map3(fn, &m[CM_PAI], v.fset[set][1], nj, ni, kz, r, l) && map3(fn, &m[CM_QSAT], v.qsat, nj, ni, kz, r, l) &&
-          map3(fn, &m[CM_ZD], v.zdiv2b, nj, ni, kz, r, l) && map3(fn, &m[CM_FMZ], v.fmz, nj, ni, kz, r, l) &&
-          map3(fn, &m[CM_T], v.t, nj, ni, kz, r, l) && map3(fn, &m[CM_QC], v.fset[set][6], nj, ni, kz, r, l) &&
-          map3(fn, &m[CM_QWL], v.qwltot, nj, ni, kz, r, l) && map3(fn, &m[CM_QWI], v.qwitot, nj, ni, kz, r, l) &&
-          map3(fn, &m[CM_S], v.s, nj, ni, kz + 1, r, l);
-      if (!ok) return false;
-    }
+  const int cols = 32 * v.twide, rows = kTwWarps / v.twide, lev = TwCfg<0>::kct;
+  auto map = [&](CUtensorMap* m, const float* base, int nk) { return map3(fn, m, base, nj, ni, nk, cols, rows, lev); };
+  for (int set = 0; set < 2; ++set) {
+    CUtensorMap* m = cm[set].m;
+    const bool ok = map(&m[CM_W], v.w, kz + 1) && map(&m[CM_FMZF], v.fmzf, kz + 1) &&
+                    map(&m[CM_QV], v.fset[set][5], kz) && map(&m[CM_TET], v.fset[set][0], kz) &&
+                    map(&m[CM_PAI], v.fset[set][1], kz) && map(&m[CM_QSAT], v.qsat, kz) &&
+                    map(&m[CM_ZD], v.zdiv2b, kz) && map(&m[CM_FMZ], v.fmz, kz) && map(&m[CM_T], v.t, kz) &&
+                    map(&m[CM_QC], v.fset[set][6], kz) && map(&m[CM_QWL], v.qwltot, kz) &&
+                    map(&m[CM_QWI], v.qwitot, kz) && map(&m[CM_S], v.s, kz + 1);
+    if (!ok) return false;
   }
   return cudaGetLastError() == cudaSuccess;
 }

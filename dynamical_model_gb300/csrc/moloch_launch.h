@@ -28,6 +28,8 @@ namespace kfast {
 int column_maps_bytes();
 // bytes of one set of tensor maps (one box shape, one buffer-set parity)
 int column_map_set_bytes();
+// warps of a column tile side by side along j, for View::twide
+int column_wide(int nj, int ni);
 bool build_column_maps(const View<float>& v, void* out);
 template <class T> int blaunch_step(const Batch<T>& b, cudaStream_t st, const PhaseFlags& fl, int& cur, int& fcur);
 template <class T> int blaunch_advection(const Batch<T>& b, cudaStream_t st, int& cur, int& fcur);

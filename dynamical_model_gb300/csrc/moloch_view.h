@@ -120,10 +120,10 @@ struct View {
   int hz_levels;
   int kmarch;      // sound kernel variants, bit mask: 1 divergence, 2 damping, 4 momentum
                    // k-marching; 8 momentum as warp strips; 16 divergence + damping fused;
-                   // 32 column solve staged by TMA with its column state in TMEM;
-                   // 64 with 8: momentum strips with two columns per lane; 128 / 256 with
-                   // 32: two words of column state a level, 12 / 16 compute warps; 512
-                   // with 16: the fused strips over two levels per warp
+                   // 32 column solve staged by TMA with its column state in TMEM (128, 256
+                   // with it: the same kernel); 64 with 8: momentum with four columns per
+                   // thread (jx a multiple of 4) or strips with two columns per lane (jx
+                   // even); 512 with 16: the fused strips over two levels per warp
   int vfields;     // advected fields per thread of k_waf_vertical: 1, 2, 5 or 10
   int srows;       // rows per warp strip of the momentum strips
   int stag4;       // 1: k_stag_from_x4 (FP32, jx a multiple of 4)
@@ -133,10 +133,11 @@ struct View {
   // accepted); nullptr when no surrogate is attached
   const int* sur_skip;
 
-  // staged column kernel (k_sound_column_tm, FP32 storage): host pointer to
+  // staged column kernel (k_sound_column_tw, FP32 storage): host pointer to
   // the two sets of TMA tensor maps (one per advected-field buffer set),
   // nullptr when the kernel cannot run on this domain
   const void* cmaps;
+  int twide;  // its warps side by side along j: tiles of 32 twide x kTwWarps / twide columns
   // device word set by a bounded wait that gave up (MOLOCH_ERR_TIMEOUT)
   int* kerr;
   long long spin_cycles;  // limit of every such wait, in SM clock cycles
@@ -192,14 +193,14 @@ struct KernelTimer {
 // rows high, given as (member, bx, 2 by8, .) so that the 32 x 4 column
 // bodies' row index by * 4 + threadIdx.y covers rows 8 by8 .. 8 by8 + 7, and
 // its strip tiles (TK_MSTRIP8, TK_DSTRIP8) are blocks of 8 warp strips.
-// TK_COLTW tiles are the 32 x kTwRows column tiles of the batched staged
-// column solve, (member, tile x, tile y, .), of the FP32 members with tensor
+// TK_COLTW tiles are the column tiles of the batched staged column solve (32
+// kTwWarps columns), (member, tile x, tile y, .), of the FP32 members with tensor
 // maps (jx a multiple of 4, kz <= 64); TK_COLREST the TK_COLUMN tiles of the
 // other members, which the one-thread column kernel takes beside it.
 // TK_DSTRIP2 tiles are blocks of 4 divergence/damping warp strips over a
 // pair of levels, (member, block, level pair, .).
 constexpr int kKC = 4;
-constexpr int kTwRows = 12;
+constexpr int kTwWarps = 8;  // compute warps (32 columns each) of a staged column tile
 constexpr int kMomJ = 30, kMomR = 32;
 constexpr int kDDJ = 29, kDDR = 32;
 constexpr int kDDLevels = 2;  // levels per warp of the two-level fused divergence/damping strips

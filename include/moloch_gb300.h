@@ -251,17 +251,16 @@ const char* moloch_gpu_kernel_name(int kind);
  *               thread, next level prefetched), 8 momentum as warp strips
  *               (30 columns x 32 rows), 16 divergence and damping fused in
  *               one warp-strip kernel (29 columns x 32 rows; overrides 1
- *               and 2; MOLOCH_FP64 ignores it), 32 the implicit-w column solve staged by TMA with
- *               its column state in TMEM (FP32 storage, jx a multiple of 4,
- *               kz <= 64; elsewhere the bit is ignored), 64 (with 8) the
- *               momentum strips with two columns per lane (62 columns x 32
- *               rows per warp, 8-byte copies; FP32 storage, jx even;
- *               elsewhere, and in ensembles, the one-column strips), 128
- *               or 256 (with 32) the staged column solve with two words of
- *               column state a level in TMEM and 12 or 16 compute warps
- *               per SM (the old w and zdiv2b staged again for the
- *               back-substitution; bit-identical to bit 32 alone; not both,
- *               and not in ensembles), 512 (with 16) the fused
+ *               and 2; MOLOCH_FP64 ignores it), 32 the implicit-w column
+ *               solve staged by TMA with its column state in TMEM (FP32
+ *               storage, jx a multiple of 4, kz <= 64; elsewhere the bit is
+ *               ignored), 64 (with 8) the momentum with four columns per
+ *               thread (FP32 storage, jx a multiple of 4) or in strips with
+ *               two columns per lane (jx even); elsewhere, and in
+ *               ensembles, the one-column strips; 128 or 256 (with 32, not
+ *               both, and not in ensembles): once other shapes of the
+ *               staged column solve, now the same kernel; 512 (with 16) the
+ *               fused
  *               divergence/damping strips over two levels per warp
  *               (shared row loads; not in ensembles); 0 = one level per
  *               thread;
