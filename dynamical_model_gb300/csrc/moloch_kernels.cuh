@@ -2078,6 +2078,238 @@ __global__ void __launch_bounds__(128, 4)
   b_divdamp_strip_nl<T, kDDLevels>(sv, t.y, t.z, R, threadIdx.x >> 5, 4);
 }
 
+// ---- divergence + divdamp with four columns per thread (FP32) ------------
+// A CTA an SM marches down the levels of tiles of 128 columns x kDQRows rows.
+// A warp per row (and one for the row on either side) holds a quad of columns
+// per lane, with u and v of the level and of the one below it in registers;
+// each level reads u, v, the v of the row after, rfw, rfs and fmz once, copied
+// kDQSlots - 1 levels ahead into a ring in shared memory (cp.async, each lane
+// its own quads); s(k+1) is carried to the next level and the 2-D metric
+// fields stay in registers.  The horizontal divergence of the rows goes
+// through shared memory (two buffers, one barrier a level); one more warp
+// forms it on the two columns beside the tile.  The tiles' levels, taken one
+// after another, are cut into one equal share a CTA, so no last wave is left.
+// Per level the arithmetic is that of b_divdamp_strip.  s is stored in the
+// last substep only (LAST): no other reads it outside this kernel.
+// The strips spend about 270 warp instructions on 32 points and issue in 60 %
+// of their cycles; this about 110.  Per step at 512 x 512 x 60: 2.32 (strips
+// over two levels) -> 1.73 ms; 10 rows 1.99, two CTAs of 5 rows 2.23; with the
+// loads in registers instead of the ring 2.15; 1024 x 1024 x 60 9.13 -> 7.35,
+// 256 x 256 x 40 0.59 -> 0.40.
+constexpr int kDQRows = 13;
+constexpr int kDQThreads = 32 * (kDQRows + 3);
+constexpr int kDQSlots = 3;
+struct DQSlot {
+  float4 f[7][32];
+  float e[2][32];  // rfw and u(k+1) of the column after the row's last
+};
+constexpr int kDQRing = (kDQRows + 2) * kDQSlots * (int)sizeof(DQSlot);
+constexpr int kDQMaxKz = 512;  // levels whose gzitak and cdamp fit beside the ring
+inline int dq_smem_bytes(int kz) { return kDQRing + 8 * kz; }
+__device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src) {
+  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(dst_smem));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+template <bool ROT, int LAST>
+__global__ void __launch_bounds__(kDQThreads, 1) k_divdamp_quad(const __grid_constant__ View<float> d) {
+  if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
+  extern __shared__ __align__(16) unsigned char dq_smem[];
+  // z of rows i0-1 .. i0+kDQRows, columns jb-4 .. jb+131 (of the outer quads only jb-1 and jb+128 are set)
+  __shared__ __align__(16) float zs[2][kDQRows + 2][136];
+  const int nj = d.nj, ni = d.ni, kz = d.kz;
+  const unsigned pl = (unsigned)d.pl;
+  const int lane = threadIdx.x, wr = threadIdx.y;
+  const int ntj = (nj + 127) / 128;
+  // gzitak(k+1), cdamp(k) behind the ring
+  float* const s_gz = reinterpret_cast<float*>(dq_smem + kDQRing);
+  float* const s_cd = s_gz + kz;
+  for (int k = lane + 32 * wr; k < kz; k += kDQThreads) { s_gz[k] = d.gzitak[k + 1]; s_cd[k] = d.cdamp[k]; }
+  const float* __restrict__ u = d.ubuf[d.cur];
+  const float* __restrict__ v = d.vbuf[d.cur];
+  const float dtrdx = d.dtrdx, dtrdy = d.dtrdy, dtrdz = d.dtrdz, ddamp2 = d.ddamp2;
+  auto zdiv = [&](float ue, float u0, float vn, float v0, float rfwe, float rfw, float rfsn, float rfs, float rmue,
+                  float rmu, float rmvn, float rmv, float fmz, float mx) {
+    if (ROT) {
+      const float du = prod_sub(dtrdx * ue, rfwe, dtrdx * u0, rfw);
+      const float dv = prod_sub((dtrdy * vn) * rfsn, rmvn, (dtrdy * v0) * rfs, rmv);
+      return (fmz * mx) * (du + dv);
+    }
+    const float du = prod_sub((dtrdx * ue) * rmue, rfwe, (dtrdx * u0) * rmu, rfw);
+    const float dv = prod_sub((dtrdy * vn) * rmvn, rfsn, (dtrdy * v0) * rmv, rfs);
+    return (mx * fmz) * (du + dv);
+  };
+  const long long total = (long long)ntj * ((ni + kDQRows - 1) / kDQRows) * kz;
+  const long long last_step = total * (blockIdx.x + 1) / gridDim.x;
+  for (long long at0 = total * blockIdx.x / gridDim.x; at0 < last_step;) {
+    const int tile = (int)(at0 / kz), k0 = (int)(at0 % kz), k1 = (int)min((long long)kz, k0 + (last_step - at0));
+    at0 += k1 - k0;
+    const int jb = tile % ntj * 128, i0 = tile / ntj * kDQRows;
+    const int rows = min(kDQRows, ni - i0);  // output rows
+    __syncthreads();  // every warp is done with the last tile's z
+    if (wr == kDQRows + 2) {
+      // the columns beside the block: lane 2 r + side
+      const int r = lane >> 1, side = lane & 1;
+      const bool on = r <= rows + 1;
+      const int jr = min(jb + 128, nj);
+      const int j = on ? (side ? (jr == nj ? 0 : jr) : (jb == 0 ? nj - 1 : jb - 1)) : 0;
+      const int i = on ? wrap2(i0 - 1 + r, ni) : 0;
+      const unsigned c = (unsigned)j + (unsigned)nj * i, ce = (unsigned)wp1(j, nj) + (unsigned)nj * i;
+      const unsigned cn = (unsigned)j + (unsigned)nj * wp1(i, ni);
+      const float mx = ROT ? d.mx[c] : d.mx2[c], rmv = d.rmv[c], rmvn = d.rmv[cn];
+      const float rmu = ROT ? 0.f : d.rmu[c], rmue = ROT ? 0.f : d.rmu[ce];
+      const int at = side ? 4 + jr - jb : 3;
+      struct E { float ue, u0, vn, v0, rfwe, rfw, rfsn, rfs, f; };
+      auto load = [&](int k, E& e) {  // the next level's, while this one's wait at the barrier
+        const unsigned o = (unsigned)k * pl;
+        e.ue = u[o + ce]; e.u0 = u[o + c]; e.vn = v[o + cn]; e.v0 = v[o + c];
+        e.rfwe = d.rfw[o + ce]; e.rfw = d.rfw[o + c]; e.rfsn = d.rfs[o + cn]; e.rfs = d.rfs[o + c]; e.f = d.fmz[o + c];
+      };
+      E e1, e2;
+      load(k0, e1);
+      if (k0 + 1 < k1) load(k0 + 1, e2);
+      for (int k = k0; k < k1; ++k) {
+        const E e = e1;
+        e1 = e2;
+        if (k + 2 < k1) load(k + 2, e2);
+        if (on) zs[k & 1][r][at] = zdiv(e.ue, e.u0, e.vn, e.v0, e.rfwe, e.rfw, e.rfsn, e.rfs, rmue, rmu, rmvn, rmv, e.f, mx);
+        __syncthreads();
+      }
+      continue;
+    }
+    // a row of quads; rows past the block's and lanes past the domain's edge only keep the barriers
+    const bool on = wr <= rows + 1, out = wr >= 1 && wr <= rows;
+    const int ii = on ? wrap2(i0 - 1 + wr, ni) : 0;
+    const int jq = jb + 4 * lane;
+    const bool in = jq < nj;
+    const int j0 = in ? jq : 0;
+    const bool endl = lane == 31 || jq + 4 >= nj;  // its east neighbours come from memory
+    const unsigned c = (unsigned)j0 + (unsigned)nj * ii, cn = (unsigned)j0 + (unsigned)nj * wp1(ii, ni);
+    const unsigned ce = (unsigned)(jq + 4 >= nj ? 0 : j0 + 4) + (unsigned)nj * ii;
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 HX = ld4(d.hx + c), HY = ld4(d.hy + c), HYN = ld4(d.hy + cn);
+    const float4 MX = ROT ? ld4(d.mx + c) : ld4(d.mx2 + c), RMV = ld4(d.rmv + c), RMVN = ld4(d.rmv + cn);
+    const float4 MU = ld4(d.mu + c), RMU = ROT ? z4 : ld4(d.rmu + c), MV = ROT ? z4 : ld4(d.mv + c);
+    // the east neighbour of a lane's last column: the lane beside, or own (a
+    // load issued together with the quads) at the end of the row
+    auto east = [&](float x, float own) {
+      const float y = __shfl_down_sync(0xffffffffu, x, 1);
+      return endl ? own : y;
+    };
+    auto own = [&](const float* p, unsigned at) { return endl ? p[at] : 0.f; };
+    const float hxe = east(HX.x, own(d.hx, ce)), rmue = ROT ? 0.f : east(RMU.x, own(d.rmu, ce));
+    // slope sums of a level pair or of one level: -> s(k) and the surface w
+    auto sval = [&](float a, float ae, float b, float bn, float hx, float hxe_, float hy, float hyn, float gz) {
+      const float zuh = prod_add(a, hx, ae, hxe_);
+      const float zvh = prod_add(b, hy, bn, hyn);
+      return -((0.25f * (zuh + zvh)) * gz);
+    };
+    auto wval = [&](float a, float ae, float b, float bn, float hx, float hxe_, float hy, float hyn) {
+      const float zuh = prod_add(a, hx, ae, hxe_);
+      const float zvh = prod_add(b, hy, bn, hyn);
+      return 0.5f * (zuh + zvh);
+    };
+    auto spair = [&](const float4& ua, float uae, const float4& ub, float ube, const float4& va, const float4& vna,
+                     const float4& vb, const float4& vnb, float gz) {  // levels a (lower) and b (upper)
+      return make_float4(
+          sval(ua.x + ub.x, ua.y + ub.y, va.x + vb.x, vna.x + vnb.x, HX.x, HX.y, HY.x, HYN.x, gz),
+          sval(ua.y + ub.y, ua.z + ub.z, va.y + vb.y, vna.y + vnb.y, HX.y, HX.z, HY.y, HYN.y, gz),
+          sval(ua.z + ub.z, ua.w + ub.w, va.z + vb.z, vna.z + vnb.z, HX.z, HX.w, HY.z, HYN.z, gz),
+          sval(ua.w + ub.w, uae + ube, va.w + vb.w, vna.w + vnb.w, HX.w, hxe, HY.w, HYN.w, gz));
+    };
+    unsigned o = (unsigned)k0 * pl;
+    float4 U = ld4(u + o + c), V = ld4(v + o + c), VN = ld4(v + o + cn);
+    float ue = own(u, o + ce);
+    ue = east(U.x, ue);
+    float4 S = z4;  // s(k)
+    if (k0 == 0) {
+      S = ld4(d.s + c);  // s at the top level is never computed here
+    } else {
+      const float4 um = ld4(u + o - pl + c), vm = ld4(v + o - pl + c), vnm = ld4(v + o - pl + cn);
+      const float ume = east(um.x, own(u, o - pl + ce));
+      S = spair(U, ue, um, ume, V, VN, vm, vnm, d.gzitak[k0]);
+    }
+    // ring of kDQSlots levels in shared memory, each lane copying and reading
+    // its own quads: rfw, rfs, rfs(i+1), fmz at k and u, v, v(i+1) at k+1
+    DQSlot* const ring = reinterpret_cast<DQSlot*>(dq_smem) + wr * kDQSlots;
+    auto issue = [&](int k) {
+      if (k < k1) {
+        DQSlot& q = ring[(k - k0) % kDQSlots];
+        const unsigned ok = (unsigned)k * pl;
+        cp_async_16(&q.f[0][lane], d.rfw + ok + c); cp_async_16(&q.f[1][lane], d.rfs + ok + c);
+        cp_async_16(&q.f[2][lane], d.rfs + ok + cn); cp_async_16(&q.f[3][lane], d.fmz + ok + c);
+        if (endl) cp_async_elem(&q.e[0][lane], d.rfw + ok + ce);
+        if (k < kz - 1) {
+          cp_async_16(&q.f[4][lane], u + ok + pl + c); cp_async_16(&q.f[5][lane], v + ok + pl + c);
+          cp_async_16(&q.f[6][lane], v + ok + pl + cn);
+          if (endl) cp_async_elem(&q.e[1][lane], u + ok + pl + ce);
+        }
+      }
+      cp_async_commit();
+    };
+  #pragma unroll
+    for (int q = 0; q < kDQSlots - 1; ++q) issue(k0 + q);
+    for (int k = k0; k < k1; ++k, o += pl) {
+      issue(k + kDQSlots - 1);  // into the slot of level k-1
+      cp_async_wait<kDQSlots - 1>();
+      const DQSlot& sl = ring[(k - k0) % kDQSlots];
+      const float4 RFW = sl.f[0][lane], RFS = sl.f[1][lane], RFSN = sl.f[2][lane], F = sl.f[3][lane];
+      float4 U1 = z4, V1 = z4, VN1 = z4;
+      if (k < kz - 1) { U1 = sl.f[4][lane]; V1 = sl.f[5][lane]; VN1 = sl.f[6][lane]; }
+      const float rfwe = east(RFW.x, sl.e[0][lane]), u1e = east(U1.x, sl.e[1][lane]);
+      float4 Z;
+      Z.x = zdiv(U.y, U.x, VN.x, V.x, RFW.y, RFW.x, RFSN.x, RFS.x, RMU.y, RMU.x, RMVN.x, RMV.x, F.x, MX.x);
+      Z.y = zdiv(U.z, U.y, VN.y, V.y, RFW.z, RFW.y, RFSN.y, RFS.y, RMU.z, RMU.y, RMVN.y, RMV.y, F.y, MX.y);
+      Z.z = zdiv(U.w, U.z, VN.z, V.z, RFW.w, RFW.z, RFSN.z, RFS.z, RMU.w, RMU.z, RMVN.z, RMV.z, F.z, MX.z);
+      Z.w = zdiv(ue, U.w, VN.w, V.w, rfwe, RFW.w, RFSN.w, RFS.w, rmue, RMU.w, RMVN.w, RMV.w, F.w, MX.w);
+      float(*const zb)[136] = zs[k & 1];
+      if (on && in) *reinterpret_cast<float4*>(&zb[wr][4 + 4 * lane]) = Z;
+      float4 S1;  // s(k+1), or -w at the surface
+      if (k < kz - 1)
+        S1 = spair(U1, u1e, U, ue, V1, VN1, V, VN, s_gz[k]);
+      else
+        S1 = make_float4(wval(U.x, U.y, V.x, VN.x, HX.x, HX.y, HY.x, HYN.x), wval(U.y, U.z, V.y, VN.y, HX.y, HX.z, HY.y, HYN.y),
+                         wval(U.z, U.w, V.z, VN.z, HX.z, HX.w, HY.z, HYN.z), wval(U.w, ue, V.w, VN.w, HX.w, hxe, HY.w, HYN.w));
+      __syncthreads();
+      if (out && in) {
+        if (k == kz - 1) {
+          st4(d.w + (unsigned)kz * pl + c, S1);
+          S1 = make_float4(-S1.x, -S1.y, -S1.z, -S1.w);
+        }
+        const float4 ZS = ld4(&zb[wr - 1][4 + 4 * lane]), ZN = ld4(&zb[wr + 1][4 + 4 * lane]);
+        const float zw = zb[wr][3 + 4 * lane], ze = zb[wr][8 + 4 * lane];
+        const float cd = s_cd[k];
+        if (LAST && k > 0) st4(d.s + o + c, S);
+        if (j0 == 0) d.eu_j[ii + (unsigned)ni * k] = U.x;
+        if (j0 + 4 == nj) d.ev_j[ii + (unsigned)ni * k] = V.w;
+        if (ii == ni - 1) st4(d.eu_i + (unsigned)nj * k + j0, U);
+        if (ii == 0) st4(d.ev_i + (unsigned)nj * k + j0, V);
+        auto un = [&](float u0, float mu, float zc, float w) { return u0 + ((cd * mu) * (zc - w)); };
+        auto vn = [&](float v0, float mv, float zc, float z0) { return ROT ? v0 + cd * (zc - z0) : v0 + ((cd * mv) * (zc - z0)); };
+        auto zn = [&](float zc, float w, float e, float z0, float z1, float fz, float s0, float s1) {
+          const float p2d = prod_sub(0.125f, ((w + e) + z0) + z1, 0.5f, zc);
+          float zd = zc + ddamp2 * p2d;
+          return zd + (fz * dtrdz) * (s0 - s1);
+        };
+        st4(d.ubuf[d.cur ^ 1] + o + c, make_float4(un(U.x, MU.x, Z.x, zw), un(U.y, MU.y, Z.y, Z.x), un(U.z, MU.z, Z.z, Z.y),
+                                                   un(U.w, MU.w, Z.w, Z.z)));
+        st4(d.vbuf[d.cur ^ 1] + o + c, make_float4(vn(V.x, MV.x, Z.x, ZS.x), vn(V.y, MV.y, Z.y, ZS.y),
+                                                   vn(V.z, MV.z, Z.z, ZS.z), vn(V.w, MV.w, Z.w, ZS.w)));
+        st4(d.zdiv2b + o + c, make_float4(zn(Z.x, zw, Z.y, ZS.x, ZN.x, F.x, S.x, S1.x), zn(Z.y, Z.x, Z.z, ZS.y, ZN.y, F.y, S.y, S1.y),
+                                          zn(Z.z, Z.y, Z.w, ZS.z, ZN.z, F.z, S.z, S1.z), zn(Z.w, Z.z, ze, ZS.w, ZN.w, F.w, S.w, S1.w)));
+      }
+      U = U1; V = V1; VN = VN1; ue = u1e; S = S1;
+    }
+    cp_async_wait<0>();  // no copy outlives the tile
+  }
+}
+
+inline bool dq_attributes() {
+  cudaFuncSetAttribute(k_divdamp_quad<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_smem_bytes(kDQMaxKz));
+  cudaFuncSetAttribute(k_divdamp_quad<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_smem_bytes(kDQMaxKz));
+  cudaFuncSetAttribute(k_divdamp_quad<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_smem_bytes(kDQMaxKz));
+  return cudaFuncSetAttribute(k_divdamp_quad<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_smem_bytes(kDQMaxKz)) == cudaSuccess;
+}
+
 // ---- advection: vertical WAF, two passes at dt/2 (:966-1073) ------------
 // wfw(k+1) of one pass from x(max(k-1,1)), x(k), x(k+1), x(min(k+2,kz))
 template <class T>
@@ -3166,7 +3398,26 @@ int launch_sound(View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
       if (d.kmarch & 16) {
         const int nstrips = ((d.nj + kDDJ - 1) / kDDJ) * ((d.ni + kDDR - 1) / kDDR);
         const dim3 g2((nstrips + 3) / 4, (d.kz + kDDLevels - 1) / kDDLevels);
-        if (d.kmarch & 512)  // kDDLevels levels per warp
+        bool quads = false;
+        if constexpr (sizeof(T) == 4) {
+          if ((d.kmarch & 512) && d.nj % 4 == 0 && d.kz <= kDQMaxKz) {  // four columns per thread
+            const int g4 = sm_count(), sm4 = dq_smem_bytes(d.kz);
+            const dim3 b4(32, kDQRows + 3);
+            static const bool attr = dq_attributes();
+            (void)attr;
+            if (d.rotllr && last)
+              MOLOCH_LAUNCH(KK_SOUND_DIVDAMP, st, k_divdamp_quad<true, 1><<<g4, b4, sm4, st>>>(d));
+            else if (d.rotllr)
+              MOLOCH_LAUNCH(KK_SOUND_DIVDAMP, st, k_divdamp_quad<true, 0><<<g4, b4, sm4, st>>>(d));
+            else if (last)
+              MOLOCH_LAUNCH(KK_SOUND_DIVDAMP, st, k_divdamp_quad<false, 1><<<g4, b4, sm4, st>>>(d));
+            else
+              MOLOCH_LAUNCH(KK_SOUND_DIVDAMP, st, k_divdamp_quad<false, 0><<<g4, b4, sm4, st>>>(d));
+            quads = true;
+          }
+        }
+        if (quads) {
+        } else if (d.kmarch & 512)  // kDDLevels levels per warp
           MOLOCH_LAUNCH(KK_SOUND_DIVDAMP, st, k_divdamp_strip_nl<T><<<g2, 128, 0, st>>>(d, kDDR));
         else
           MOLOCH_LAUNCH(KK_SOUND_DIVDAMP, st, k_divdamp_strip<T><<<dim3((nstrips + 3) / 4, d.kz), 128, 0, st>>>(d, kDDR));
