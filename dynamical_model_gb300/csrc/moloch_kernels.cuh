@@ -474,9 +474,7 @@ __device__ __forceinline__ T zrom1w_moist(T zrom1w, T qvk, T qsk, T qskm, T wk, 
 // measured 13 % slower at 512 x 512 x 60: fewer columns in flight cost more
 // bandwidth than the extra L2 hits saved.
 template <class T, int PD>
-__device__ __forceinline__ void b_sound_column_std(const View<T>& d, const int bx, const int by, int nsound, int last, int defer_pai) {
-  const int jj = bx * kColBX + threadIdx.x;
-  const int ii = by * kColBY + threadIdx.y;
+__device__ __forceinline__ void b_sound_column_std(const View<T>& d, const int jj, const int ii, int nsound, int last, int defer_pai) {
   const int nj = d.nj, ni = d.ni, kz = d.kz;
   if (jj >= nj || ii >= ni) return;
   const size_t pl = d.pl;
@@ -667,10 +665,8 @@ __device__ __forceinline__ void b_sound_column_std(const View<T>& d, const int b
 // doubles order as their bits) before it forms anything.
 // 256 x 256 x 60: 8.6 -> 5.1 ms per step (84 % of the FP64 pipe).
 template <int PD>
-__device__ __forceinline__ void b_sound_column_lean(const View<double>& d, const int bx, const int by, int nsound,
+__device__ __forceinline__ void b_sound_column_lean(const View<double>& d, const int jj, const int ii, int nsound,
                                                     int last, int defer_pai) {
-  const int jj = bx * kColBX + threadIdx.x;
-  const int ii = by * kColBY + threadIdx.y;
   const int nj = d.nj, ni = d.ni, kz = d.kz;
   if (jj >= nj || ii >= ni) return;
   const size_t pl = d.pl;
@@ -804,18 +800,30 @@ __device__ __forceinline__ void b_sound_column_lean(const View<double>& d, const
 }
 
 template <class T, int PD>
-__device__ __forceinline__ void b_sound_column(const View<T>& d, const int bx, const int by, const int bz, int nsound, int last, int defer_pai) {
+__device__ __forceinline__ void b_sound_column(const View<T>& d, const int jj, const int ii, int nsound, int last,
+                                               int defer_pai) {
   if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
-  if constexpr (kLean<T>) b_sound_column_lean<PD>(d, bx, by, nsound, last, defer_pai);
-  else b_sound_column_std<T, PD>(d, bx, by, nsound, last, defer_pai);
+  if constexpr (kLean<T>) b_sound_column_lean<PD>(d, jj, ii, nsound, last, defer_pai);
+  else b_sound_column_std<T, PD>(d, jj, ii, nsound, last, defer_pai);
 }
 
 // FP32: 9 blocks of 128 threads per SM (56 registers, 24 bytes spilled):
 // 1.5 waves at 512 x 512 instead of 1.68 with 8 blocks (4.51 against
 // 4.61 ms per step; 10 blocks, 48 registers, 4.84 ms)
-template <class T>
-__global__ void __launch_bounds__(kColBX* kColBY, sizeof(T) == 4 ? 9 : 4) k_sound_column(View<T> d, int nsound, int last, int defer_pai) {
-  b_sound_column<T, 1>(d, blockIdx.x, blockIdx.y, blockIdx.z, nsound, last, defer_pai);
+//
+// PD = 2, 4 blocks (118 registers): the FP32 kernel of domains whose columns
+// (up to 4 x 128 x SMs) are all in flight at once either way, where a second
+// level of loads in flight hides more than occupancy does: 28 against 35 us
+// per launch at 100 x 100 x 30, 56 against 75 at 203 x 157 x 45, 64 against 80
+// at 256 x 256 x 40; above, 188 against 172 at 384 x 384 x 60.  FP64 gains
+// nothing from it (81 against 82 us at 100 x 100 x 30).  Where blocks of four
+// rows are fewer than two an SM, blocks of one row spread the warps: exact
+// FP64 at 100 x 100 x 30 115 -> 105 us.
+template <class T, int PD>
+__global__ void __launch_bounds__(kColBX* kColBY, sizeof(T) == 4 && PD == 1 ? 9 : 4)
+    k_sound_column(View<T> d, int nsound, int last, int defer_pai) {
+  b_sound_column<T, PD>(d, blockIdx.x * kColBX + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, nsound, last,
+                        defer_pai);
 }
 
 template <class T>
@@ -825,7 +833,7 @@ __global__ void __launch_bounds__(kColBX* kColBY, sizeof(T) == 4 ? 8 : 4)
   const int4 t = tiles[blockIdx.x];
   copy_view(&sv, views + t.x);
   __syncthreads();
-  b_sound_column<T, 1>(sv, t.y, t.z, t.w, nsound, last, defer_pai);
+  b_sound_column<T, 1>(sv, t.y * kColBX + threadIdx.x, t.z * kColBY + threadIdx.y, nsound, last, defer_pai);
 }
 
 
@@ -3199,47 +3207,47 @@ __global__ void __launch_bounds__(kPtBX* kPtBY)
 }
 
 
-// ---- post-diagnostics (:355-391), one thread per column ----------------
+// ---- post-diagnostics (:355-391), one thread per point -------------------
+// The threads of the lowest level also form the surface pressure, from tvirt
+// of the two lowest levels.  One thread per column marched down the levels
+// with one level of loads in flight: 100 x 100 x 30 FP32 33 -> 8 us, FP64 88 ->
+// 46, 256 x 256 x 40 FP32 66 -> 31; 512 x 512 x 60 the same 0.145 ms.
 template <class T>
-__device__ __forceinline__ void b_postdiag(const View<T>& d, const int bx, const int by, const int bz) {  const T* __restrict__ zk = d.zeta + (size_t)d.pl * (d.kz - 1);
-  const T* __restrict__ zkm1 = d.zeta + (size_t)d.pl * (d.kz - 2);
-
-  int jj = bx * kColBX + threadIdx.x;
-  int ii = by * kColBY + threadIdx.y;
+__device__ __forceinline__ void b_postdiag(const View<T>& d, const int bx, const int by, const int bz) {
+  const int jj = bx * kPtBX + threadIdx.x;
+  const int ii = by * kPtBY + threadIdx.y;
   const int nj = d.nj, ni = d.ni, kz = d.kz;
   if (jj >= nj || ii >= ni) return;
   const size_t pl = d.pl;
   const size_t c = jj + (size_t)nj * ii;
-  T tv_km1 = T(0), tv_k = T(0), p_k = T(0);
-  for (int kk = 0; kk < kz; ++kk) {
-    const size_t q = c + (size_t)kk * pl;
-    const T pai = d.pai[q];
-    const T tv = d.tetav[q] * pai;
-    d.tvirt[q] = tv;
-    const T qv = d.q[0][q], qc = d.q[1][q], qi = d.q[2][q], qr = d.q[3][q], qs = d.q[4][q];
-    const T t = ddiv(tv, (((T(1) + T(kEp1) * qv) - qc) - qi) - qr - qs);
-    d.t[q] = t;
-    const T p = pow_cpovr(pai) * T(kP00);
-    d.p[q] = p;
-    d.rho[q] = ddiv(p, T(kRgas) * t);
-    d.qsat[q] = pfwsat(t, p);
-    tv_km1 = tv_k; tv_k = tv; p_k = p;
-  }
-  const T z = zk[c], zm = zkm1[c];
+  const size_t q = c + (size_t)bz * pl;
+  const T pai = d.pai[q];
+  const T tvk = mul_rn(d.tetav[q], pai);  // rounded products, also inside the lapse rate below
+  d.tvirt[q] = tvk;
+  const T qv = d.q[0][q], qc = d.q[1][q], qi = d.q[2][q], qr = d.q[3][q], qs = d.q[4][q];
+  const T t = ddiv(tvk, (((T(1) + T(kEp1) * qv) - qc) - qi) - qr - qs);
+  d.t[q] = t;
+  const T p = pow_cpovr(pai) * T(kP00);
+  d.p[q] = p;
+  d.rho[q] = ddiv(p, T(kRgas) * t);
+  d.qsat[q] = pfwsat(t, p);
+  if (bz != kz - 1) return;
+  const T tv_km1 = mul_rn(d.tetav[q - pl], d.pai[q - pl]);
+  const T z = d.zeta[q], zm = d.zeta[q - pl];
   const T zdgz = z * T(kEgrav);
-  T lrt = (tv_km1 - tv_k) / (zm - z);
+  T lrt = (tv_km1 - tvk) / (zm - z);
   lrt = T(0.65) * lrt - T(0.35) * T(kLrate);
-  const T tv = tv_k - (T(0.5) * z) * lrt;
-  d.ps[c] = p_k * dexp(zdgz / (T(kRgas) * tv));
+  const T tv = tvk - (T(0.5) * z) * lrt;
+  d.ps[c] = p * dexp(zdgz / (T(kRgas) * tv));
 }
 
 template <class T>
-__global__ void __launch_bounds__(kColBX* kColBY) k_postdiag(View<T> d) {
+__global__ void __launch_bounds__(kPtBX* kPtBY) k_postdiag(View<T> d) {
   b_postdiag<T>(d, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 template <class T>
-__global__ void __launch_bounds__(kColBX* kColBY)
+__global__ void __launch_bounds__(kPtBX* kPtBY)
     kb_postdiag(const View<T>* __restrict__ views, const int4* __restrict__ tiles) {
   __shared__ View<T> sv;
   const int4 t = tiles[blockIdx.x];
@@ -3369,6 +3377,21 @@ inline int sm_count() {
   }
   return nsm;
 }
+// the one-thread column solve (variants: k_sound_column)
+template <class T>
+void launch_sound_column(const View<T>& d, cudaStream_t st, int ns, int last, int defer_pai) {
+  const int bj = (d.nj + kColBX - 1) / kColBX;
+  const int rows = bj * ((d.ni + kColBY - 1) / kColBY) < 2 * sm_count() ? 1 : kColBY;
+  const dim3 cb(kColBX, rows), cg(bj, (d.ni + rows - 1) / rows);
+  if constexpr (sizeof(T) == 4) {
+    if (d.pl <= 4 * kColBX * kColBY * sm_count()) {
+      MOLOCH_LAUNCH(KK_SOUND_COLUMN, st, k_sound_column<T, 2><<<cg, cb, 0, st>>>(d, ns, last, defer_pai));
+      return;
+    }
+  }
+  MOLOCH_LAUNCH(KK_SOUND_COLUMN, st, k_sound_column<T, 1><<<cg, cb, 0, st>>>(d, ns, last, defer_pai));
+}
+
 // persistent CTAs of the staged column solve over ntiles tiles
 inline int column_tw_grid(int ntiles) {
   const int slots = TwCfg<0>::ctas * sm_count();
@@ -3385,7 +3408,6 @@ inline int column_tw_grid(const View<T>& d) {
 template <class T>
 int launch_sound(View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
   int n = 0;
-  const dim3 cb(kColBX, kColBY), cg = col_grid(d.nj, d.ni);
   const dim3 pb(kPtBX, kPtBY), pg = pt_grid(d.nj, d.ni, d.kz);
   const dim3 kg = pt_grid(d.nj, d.ni, (d.kz + kKC - 1) / kKC);  // k-marching: chunks of kKC levels
   for (int ns = 1; ns <= fl.nsound; ++ns) {
@@ -3438,7 +3460,7 @@ int launch_sound(View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
       n += 2;
     }
     if (fl.divfilter) {
-      MOLOCH_LAUNCH(KK_SOUND_COLUMN, st, k_sound_column<T><<<cg, cb, 0, st>>>(d, ns, last, 1));
+      launch_sound_column<T>(d, st, ns, last, 1);
       MOLOCH_LAUNCH(KK_LAP_FILTER, st, k_lap_filter<T><<<pg, pb, 0, st>>>(d));
       MOLOCH_LAUNCH(KK_PAI_UPDATE, st, k_pai_update<T><<<pg, pb, 0, st>>>(d));
       n += 3;
@@ -3457,7 +3479,7 @@ int launch_sound(View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
           staged = true;
         }
       }
-      if (!staged) MOLOCH_LAUNCH(KK_SOUND_COLUMN, st, k_sound_column<T><<<cg, cb, 0, st>>>(d, ns, last, 0));
+      if (!staged) launch_sound_column<T>(d, st, ns, last, 0);
       ++n;
     }
     bool pairs = false;
@@ -3556,7 +3578,7 @@ int launch_postdiag(View<T>& d, cudaStream_t st, const PhaseFlags& fl, const T* 
     cudaMemcpyAsync(d.tetav, d.fscr, bytes, cudaMemcpyDeviceToDevice, st);
     ++n;
   }
-  MOLOCH_LAUNCH(KK_POSTDIAG, st, k_postdiag<T><<<col_grid(d.nj, d.ni), dim3(kColBX, kColBY), 0, st>>>(d));
+  MOLOCH_LAUNCH(KK_POSTDIAG, st, k_postdiag<T><<<pg, pb, 0, st>>>(d));
   return n + 1;
 }
 
@@ -3666,7 +3688,7 @@ int blaunch_step(const Batch<T>& b, cudaStream_t st, const PhaseFlags& fl, int& 
     cur = 0;
     n += 3;
   }
-  MOLOCH_LAUNCH(KK_POSTDIAG, st, kb_postdiag<T><<<nco, cb, 0, st>>>(V(), CO));
+  MOLOCH_LAUNCH(KK_POSTDIAG, st, kb_postdiag<T><<<npt, pb, 0, st>>>(V(), PT));
   return n + 1;
 }
 

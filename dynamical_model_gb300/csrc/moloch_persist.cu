@@ -54,7 +54,7 @@ __device__ __forceinline__ void run_item(const View<T>& d, const Phase& ph, cons
     case PH_DIV_KM: b_sound_div_km<T>(d, t.y, t.z, t.w); break;
     case PH_DAMP: b_sound_damp<T>(d, t.y, t.z, t.w); break;
     case PH_DAMP_KM: b_sound_damp_km<T>(d, t.y, t.z, t.w); break;
-    case PH_COLUMN: b_sound_column<T, 1>(d, t.y, t.z, t.w, ph.a0, ph.a1, ph.a2); break;
+    case PH_COLUMN: b_sound_column<T, 1>(d, t.y * kColBX + threadIdx.x, t.z * kColBY + threadIdx.y, ph.a0, ph.a1, ph.a2); break;
     case PH_LAP_FILTER: b_lap_filter<T>(d, t.y, t.z, t.w); break;
     case PH_PAI_UPDATE: b_pai_update<T>(d, t.y, t.z, t.w); break;
     case PH_MOM_STRIP: b_momentum_strip<T>(d, t.y, t.z, ph.a0, ring[threadIdx.y], threadIdx.y, kWarps); break;
@@ -209,7 +209,7 @@ int program(const Batch<T>& b, const PhaseFlags& fl, int fcur, int grid, std::ve
     P(PH_STAG, TK_POINT);
     cur = 0;
   }
-  P(PH_POSTDIAG, TK_COLUMN8);
+  P(PH_POSTDIAG, TK_POINT);
   return (int)out.size() <= kMaxPhases ? 0 : 2;
 }
 
