@@ -269,6 +269,52 @@ PhaseFlags flags_of(const moloch_handle* h) {
   return f;
 }
 
+// Launch shapes of a handle nothing else was chosen for (moloch_gpu_set_tuning
+// and moloch_gpu_autotune override them), by the size of the domain.  Every
+// variant named here gives the bits of one level, field and tile level a
+// thread.  us per launch, first the shape up to that size, then the one above
+// it:
+//   FP32, jx a multiple of 4 (quads, staged column solve, 16-byte staggering):
+//     divergence + damping 17 | 11 at 100 x 100 x 30, 48 | 26 at 256 x 256 x 40;
+//     momentum 10 | 8 and 39 | 20; column solve 28 | 26 and 64 | 47
+//   FP32, other jx, 203 x 157 x 45: divergence + damping 34 | 30 (fused strips,
+//     one launch less), momentum 25 | 22; at 64 x 64 x 30 the strips lose (13 |
+//     21, 8 | 9), so they start at 2^20 points
+//   horizontal WAF, tiles | strips of 16 rows: FP32 27 | 29 at 64 x 64 x 30, 52 |
+//     33 at 100 x 100 x 30, 289 | 111 at 256 x 256 x 40; FP64 71 | 123, 193 | 183,
+//     1073 | 1063; strips of 32 rows from 512 x 512 in FP32 (586 | 565 at
+//     512 x 512 x 60) and 256 x 256 in FP64 (1420 | 1395 at 256 x 256 x 60)
+//   vertical WAF, FP64, fields a thread 1 | 2 | 5: 43 | 45 | 83 at 48 x 40 x 20,
+//     186 | 164 | 178 at 100 x 100 x 30, 660 | 609 | 550 at 203 x 157 x 45
+//   FP64 divergence, damping, momentum, a level a thread | k-marching: 18, 18,
+//     35 | 18, 18, 39 at 100 x 100 x 30; 53, 53, 121 | 49, 45, 109 at 203 x 157 x 45
+// The exact build keeps one level, field and tile level a thread (823 us of
+// tiles | 1124 of strips at 100 x 100 x 30).
+template <class T>
+void default_shapes(View<T>& v, int mode) {
+  const long cols = (long)v.nj * v.ni, pts = cols * v.kz;
+  v.hz_levels = 1;
+  v.kmarch = 0;
+  v.vfields = 1;
+  v.srows = kMomR;
+  v.stag4 = 0;
+  v.cor_rounded = 1;
+  if (mode == MOLOCH_FP32_MIXED) {
+    v.srows = 8;
+    if (pts >= 200000) v.hz_levels = cols >= 200000 ? 32 : 16;
+    if (v.nj % 4 == 0) {
+      v.kmarch = 16 | 512 | 32 | 128 | 8 | 64;
+      v.stag4 = 1;
+    } else if (pts >= 1 << 20) {
+      v.kmarch = 16 | 8 | 64;
+    }
+  } else if (mode == MOLOCH_FP64) {
+    if (cols >= 8000) v.hz_levels = cols >= 60000 ? 32 : 16;
+    v.vfields = cols >= 20000 ? 5 : cols >= 4000 ? 2 : 1;
+    if (cols >= 20000) v.kmarch = 1 | 2 | 4;
+  }
+}
+
 // carve the arena; returns bytes needed when base == nullptr
 template <class T>
 size_t layout(View<T>& v, char* base, const moloch_handle* h) {
@@ -318,11 +364,7 @@ size_t layout(View<T>& v, char* base, const moloch_handle* h) {
   v.dparts = parts;
   v.nj = h->nj(); v.ni = h->ni(); v.kz = h->kz(); v.pl = (int)pl; v.rotllr = h->prm.rotllr;
   v.cur = 0;
-  v.hz_levels = 1;
-  v.kmarch = 0;
-  v.vfields = 1;
-  v.srows = kMomR;
-  v.stag4 = 0;
+  default_shapes(v, h->prm.mode);
   v.sur_skip = nullptr;
   v.cmaps = nullptr;
   v.twide = 1;
@@ -1403,7 +1445,11 @@ int moloch_gpu_set_tuning(moloch_handle_t* h, const int* choice, int n) {
     return fail(MOLOCH_ERR_ARG, "rows per momentum strip %d", choice[3]);
   if (n > 4 && (choice[4] < 0 || choice[4] > 1)) return fail(MOLOCH_ERR_ARG, "staggering variant %d", choice[4]);
   if (n > 0) { h->vd.hz_levels = choice[0]; h->vf.hz_levels = choice[0]; }
-  if (n > 1) { h->vd.kmarch = choice[1]; h->vf.kmarch = choice[1]; }
+  if (n > 1) {
+    h->vd.kmarch = choice[1];
+    h->vf.kmarch = choice[1];
+    h->vd.cor_rounded = h->vf.cor_rounded = 0;
+  }
   if (n > 2) { h->vd.vfields = choice[2]; h->vf.vfields = choice[2]; }
   if (n > 3) { h->vd.srows = choice[3]; h->vf.srows = choice[3]; }
   if (n > 4) { h->vd.stag4 = choice[4]; h->vf.stag4 = choice[4]; }
@@ -1579,6 +1625,7 @@ struct moloch_ensemble {
   int kmarch = 0;
   int vfields = 1;
   int mrows = kMomR;  // rows per momentum warp strip of the one-launch-per-kernel mode
+  bool tuned = false;  // shapes given by the caller or the autotuner; else by ens_default_shapes
   int cur = 0, fcur = 0;
   long long kernels = 0;
   int kernels_per_step = 0;
@@ -1704,6 +1751,7 @@ int ens_upload(moloch_ensemble* e, Batch<T>& b, View<T> moloch_handle::*vm) {
         v.fcur = fc;
         v.hz_levels = e->hz_levels >= 16 ? e->hz_levels : std::min(e->hz_levels, v.kz);
         v.vfields = e->vfields;
+        v.cor_rounded = e->tuned ? 0 : 1;
         v.bind_fields();
         hv[(size_t)(cur * 2 + fc) * n + q] = v;
       }
@@ -1764,7 +1812,24 @@ int ens_upload(moloch_ensemble* e, Batch<T>& b, View<T> moloch_handle::*vm) {
   return MOLOCH_OK;
 }
 
+// Launch shapes of an ensemble nothing else was chosen for.  From 2^20 points
+// on (12 uneven members of 10.5 M points, ms per step: horizontal WAF tiles of
+// four levels 3.64, strips of 32 rows 1.36; FP32 divergence and damping a level
+// a thread 3.46, fused strips over two levels 1.93; momentum 3.12, strips 1.67;
+// FP64 as in default_shapes) the variants of larger domains, below and in
+// persistent mode the shapes the persistent kernel carries.
+void ens_default_shapes(moloch_ensemble* e, bool persistent) {
+  long pts = 0;
+  for (auto* h : e->m) pts += (long)h->nj() * h->ni() * h->kz();
+  const bool large = pts >= 1 << 20 && !persistent;
+  e->hz_levels = large ? (e->elem == 4 ? 32 : 16) : 4;
+  e->kmarch = !large ? 0 : e->elem == 8 ? 1 | 2 | 4 : 16 | 512 | 8;
+  e->vfields = large && e->elem == 8 ? 2 : 1;
+  e->mrows = kMomR;
+}
+
 int ens_build(moloch_ensemble* e) {
+  if (!e->tuned) ens_default_shapes(e, e->persistent != 0);
   ens_drop_graphs(e);
   ens_tiles(e);
   return e->elem == 8 ? ens_upload(e, e->bd, &moloch_handle::vd) : ens_upload(e, e->bf, &moloch_handle::vf);
@@ -1886,6 +1951,8 @@ int moloch_gpu_ensemble_autotune(moloch_ensemble_t* e, int* choice, double* best
   cudaEvent_t e0, e1;
   CUDA_TRY(cudaEventCreate(&e0));
   CUDA_TRY(cudaEventCreate(&e1));
+  if (!e->tuned) ens_default_shapes(e, true);  // the base shapes
+  e->tuned = true;
   double best = 1e30;
   int pick = e->hz_levels;
   for (int c = 0; c < 7; ++c) {
@@ -2065,6 +2132,8 @@ int moloch_gpu_ensemble_set_tuning(moloch_ensemble_t* e, const int* choice, int 
   if (nchoice > 3 && (choice[3] < 4 || choice[3] > 64))
     return fail(MOLOCH_ERR_ARG, "rows per momentum strip %d", choice[3]);
   if (nchoice > 4 && (choice[4] < 0 || choice[4] > 1)) return fail(MOLOCH_ERR_ARG, "staggering variant %d", choice[4]);
+  if (!e->tuned) ens_default_shapes(e, true);  // slots not given: the base shapes
+  e->tuned = true;
   if (nchoice > 0) e->hz_levels = choice[0];
   if (nchoice > 1) e->kmarch = choice[1];
   if (nchoice > 2) e->vfields = choice[2];
@@ -2078,6 +2147,7 @@ int moloch_gpu_ensemble_set_persistent(moloch_ensemble_t* e, int on) {
   g_err.clear();
   if (!e) return fail(MOLOCH_ERR_ARG, "null ensemble");
   if (on < 0 || on > 4) return fail(MOLOCH_ERR_ARG, "persistent %d: 0 off, 1 default, 2-4 blocks per SM", on);
+  if (!e->tuned) ens_default_shapes(e, on != 0);
   if (on) {
     const bool ok = e->elem == 8 ? persist::supports<double>(e->hz_levels, e->kmarch, e->vfields)
                                  : persist::supports<float>(e->hz_levels, e->kmarch, e->vfields);

@@ -955,6 +955,17 @@ __global__ void __launch_bounds__(kPtBX* kPtBY)
 }
 
 
+// u plus and v minus the Coriolis term k sum of Equations 17 and 18.  FP32: as
+// one multiply-add, or (rounded) with the product rounded first, as
+// k_sound_momentum takes it; the rest of the equations rounds alike in all
+// variants.  The quads and strips can do either (View::cor_rounded).
+__device__ __forceinline__ float plus_cor(float u, float k, float sum, int rounded) {
+  return rounded ? __fadd_rn(u, __fmul_rn(k, sum)) : __fmaf_rn(k, sum, u);
+}
+__device__ __forceinline__ double plus_cor(double u, double k, double sum, int) { return u + k * sum; }
+template <class T>
+__device__ __forceinline__ T minus_cor(T v, T k, T sum, int rounded) { return plus_cor(v, -k, sum, rounded); }
+
 // ---- sound: momentum, Equations 17 and 18 (:737-837) --------------------
 // One thread per point; reads u, v (current buffer, damped interior + the
 // pre-damping edges) and writes the other buffer of the pair.
@@ -992,9 +1003,9 @@ __device__ __forceinline__ void b_sound_momentum(const View<T>& d, const int bx,
     const T vdw = jj == 0 ? d.ev_j[ii + (size_t)ni * kk] : v[cw + o];
     const T vdwn = jj == 0 ? d.ev_j[ip + (size_t)ni * kk] : (ii == ni - 1 ? d.ev_i[jm + (size_t)nj * kk] : v[cwn + o]);
     const T vdn = ii == ni - 1 ? d.ev_i[jj + (size_t)nj * kk] : v[cn + o];
-    const T zcor1u = ((d.coru[c] * dts) * T(0.25)) * (((vdc + vdw) + vdwn) + vdn);
+    const T ucor = plus_cor(u[c + o], (d.coru[c] * dts) * T(0.25), ((vdc + vdw) + vdwn) + vdn, 1);
     const T paw = jj == 0 ? d.ep_j[ii + (size_t)ni * kk] : d.pai[cw + o];
-    uo[c + o] = ((u[c + o] + zcor1u) - (zfz * d.hx[c]) * gzh) - (zcx * zrom1u) * (pc - paw);
+    uo[c + o] = (ucor - (zfz * d.hx[c]) * gzh) - (zcx * zrom1u) * (pc - paw);
   }
   // Equation 18
   {
@@ -1005,9 +1016,9 @@ __device__ __forceinline__ void b_sound_momentum(const View<T>& d, const int bx,
     const T uds = ii == 0 ? d.eu_i[jj + (size_t)nj * kk] : u[cs + o];
     const T ude = jj == nj - 1 ? d.eu_j[ii + (size_t)ni * kk] : u[ce + o];
     const T udes = jj == nj - 1 ? d.eu_j[im + (size_t)ni * kk] : (ii == 0 ? d.eu_i[jp + (size_t)nj * kk] : u[ces + o]);
-    const T zcor1v = ((d.corv[c] * dts) * T(0.25)) * (((udc + uds) + ude) + udes);
+    const T vcor = minus_cor(v[c + o], (d.corv[c] * dts) * T(0.25), ((udc + uds) + ude) + udes, 1);
     const T pas = ii == 0 ? d.ep_i[jj + (size_t)nj * kk] : d.pai[cs + o];
-    vo[c + o] = ((v[c + o] - zcor1v) - (zfz * d.hy[c]) * gzh) - (zcy * zrom1v) * (pc - pas);
+    vo[c + o] = (vcor - (zfz * d.hy[c]) * gzh) - (zcy * zrom1v) * (pc - pas);
   }
 }
 
@@ -1244,15 +1255,15 @@ __device__ __forceinline__ void b_sound_momentum_km(const View<T>& d, const int 
     {
       const T zfz = egdts + T(0.25) * (((dw_w + cur.dww1) + dw_c) + cur.dwc1);
       const T zrom1u = hcpd * (cur.tw + tc);
-      const T zcor1u = corx * (((cur.vc + cur.vw) + cur.vwn) + cur.vn);
-      uo[c + o] = ((cur.uc + zcor1u) - (zfz * hxc) * gzh) - (zcx * zrom1u) * (pc - cur.pw);
+      const T ucor = plus_cor(cur.uc, corx, ((cur.vc + cur.vw) + cur.vwn) + cur.vn, 0);
+      uo[c + o] = (ucor - (zfz * hxc) * gzh) - (zcx * zrom1u) * (pc - cur.pw);
     }
     // Equation 18
     {
       const T zfz = egdts + T(0.25) * (((dw_s + cur.dws1) + dw_c) + cur.dwc1);
       const T zrom1v = hcpd * (cur.ts + tc);
-      const T zcor1v = cory * (((cur.uc + cur.us) + cur.ue) + cur.ues);
-      vo[c + o] = ((cur.vc - zcor1v) - (zfz * hyc) * gzh) - (zcy * zrom1v) * (pc - cur.ps);
+      const T vcor = minus_cor(cur.vc, cory, ((cur.uc + cur.us) + cur.ue) + cur.ues, 0);
+      vo[c + o] = (vcor - (zfz * hyc) * gzh) - (zcy * zrom1v) * (pc - cur.ps);
     }
     dw_c = cur.dwc1; dw_w = cur.dww1; dw_s = cur.dws1;
   }
@@ -1337,6 +1348,7 @@ __device__ __forceinline__ void b_momentum_strip(const View<T>& d, const int bx,
   const T hcpd = T(0.5) * T(kCpd);
   const T gzh = d.gzitakh[k];
   const bool rot = d.rotllr;
+  const int rounded = d.cor_rounded;
   const int jm = wm1(jj, nj), jp = wp1(jj, nj);
   // rows i_s-1 .. i_e stream through the slots in order; the slot indices
   // rotate by one per row
@@ -1410,8 +1422,8 @@ __device__ __forceinline__ void b_momentum_strip(const View<T>& d, const int bx,
           vdn = ii == ni - 1 ? d.ev_i[jj + (size_t)nj * k] : vn;
           paw = jj == 0 ? d.ep_j[ii + (size_t)ni * k] : pw;
         }
-        const T zcor1u = ((c2.coru * dts) * T(0.25)) * (((vdc + vdw) + vdwn) + vdn);
-        uo[(size_t)jj + (size_t)nj * ii] = ((cu + zcor1u) - (zfz * c2.hx) * gzh) - (zcx * zrom1u) * (pc - paw);
+        const T ucor = plus_cor(cu, (c2.coru * dts) * T(0.25), ((vdc + vdw) + vdwn) + vdn, rounded);
+        uo[(size_t)jj + (size_t)nj * ii] = (ucor - (zfz * c2.hx) * gzh) - (zcx * zrom1u) * (pc - paw);
       }
       // Equation 18
       {
@@ -1427,8 +1439,8 @@ __device__ __forceinline__ void b_momentum_strip(const View<T>& d, const int bx,
           udes = jj == nj - 1 ? d.eu_j[im + (size_t)ni * k] : (ii == 0 ? d.eu_i[jp + (size_t)nj * k] : ues);
           pas = ii == 0 ? d.ep_i[jj + (size_t)nj * k] : ps;
         }
-        const T zcor1v = ((c2.corv * dts) * T(0.25)) * (((udc + uds) + ude) + udes);
-        vo[(size_t)jj + (size_t)nj * ii] = ((cv - zcor1v) - (zfz * c2.hy) * gzh) - (zcy * zrom1v) * (pc - pas);
+        const T vcor = minus_cor(cv, (c2.corv * dts) * T(0.25), ((udc + uds) + ude) + udes, rounded);
+        vo[(size_t)jj + (size_t)nj * ii] = (vcor - (zfz * c2.hy) * gzh) - (zcy * zrom1v) * (pc - pas);
       }
     }
     qb = qc; qc = qn; qn = nxt(qn); qi = nxt(qi);
@@ -1505,6 +1517,7 @@ __device__ __forceinline__ void b_momentum_strip2(const View<float>& d, const in
   const float hcpd = 0.5f * float(kCpd);
   const float gzh = d.gzitakh[k];
   const bool rot = d.rotllr;
+  const int rounded = d.cor_rounded;
   auto nxt = [](int q) { return q + 1 == kMom2S ? 0 : q + 1; };
   auto issue = [&](int r, int q) {  // copies of row r into slot q (nothing past i_e); one group either way
     if (r <= i_e) {
@@ -1552,8 +1565,8 @@ __device__ __forceinline__ void b_momentum_strip2(const View<float>& d, const in
         vdn = ii == ni - 1 ? d.ev_i[jj + (size_t)nj * k] : x.vn;
         paw = jj == 0 ? d.ep_j[ii + (size_t)ni * k] : pw;
       }
-      const float zcor1u = ((coru * dts) * 0.25f) * (((x.cv + vdw) + vdwn) + vdn);
-      un = ((x.cu + zcor1u) - (zfz * hx) * gzh) - (zcx * zrom1u) * (x.cp - paw);
+      const float ucor = plus_cor(x.cu, (coru * dts) * 0.25f, ((x.cv + vdw) + vdwn) + vdn, rounded);
+      un = (ucor - (zfz * hx) * gzh) - (zcx * zrom1u) * (x.cp - paw);
     }
     // Equation 18
     {
@@ -1568,8 +1581,8 @@ __device__ __forceinline__ void b_momentum_strip2(const View<float>& d, const in
         udes = jj == nj - 1 ? d.eu_j[im + (size_t)ni * k] : (ii == 0 ? d.eu_i[jp + (size_t)nj * k] : ues);
         pas = ii == 0 ? d.ep_i[jj + (size_t)nj * k] : x.ps;
       }
-      const float zcor1v = ((corv * dts) * 0.25f) * (((x.cu + uds) + ude) + udes);
-      vnew = ((x.cv - zcor1v) - (zfz * hy) * gzh) - (zcy * zrom1v) * (x.cp - pas);
+      const float vcor = minus_cor(x.cv, (corv * dts) * 0.25f, ((x.cu + uds) + ude) + udes, rounded);
+      vnew = (vcor - (zfz * hy) * gzh) - (zcy * zrom1v) * (x.cp - pas);
     }
   };
   auto row = [&](const int i, auto edge) {
@@ -1662,6 +1675,7 @@ __global__ void __launch_bounds__(32 * kQuadY, 5) k_momentum_quad(const __grid_c
   const float4 CU = ld4(d.coru + r + j0), CV = ld4(d.corv + r + j0), HX = ld4(d.hx + r + j0), HY = ld4(d.hy + r + j0);
   const float4 MU = ld4(d.mu + r + j0);
   const bool rot = d.rotllr;
+  const int rounded = d.cor_rounded;
   const float4 MV = rot ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4(d.mv + r + j0);
   // column j0-1 of v, v(i+1), tetav, pai, deltaw and column j0+4 of u, u(i-1)
   float vw = 0.f, vnw = 0.f, tw = 0.f, pw = 0.f, dw0 = 0.f, dw1 = 0.f, ue = 0.f, use = 0.f;
@@ -1699,16 +1713,16 @@ __global__ void __launch_bounds__(32 * kQuadY, 5) k_momentum_quad(const __grid_c
     const float zcx = dtrdx * mu;
     const float zfz = egdts + 0.25f * (((wd0 + wd1) + cd0) + cd1);
     const float zrom1u = hcpd * (wt + ct);
-    const float zcor1u = ((coru * dts) * 0.25f) * (((cv + wv) + wvn) + cvn);
-    return ((cu + zcor1u) - (zfz * hx) * gzh) - (zcx * zrom1u) * (cp - wp);
+    const float ucor = plus_cor(cu, (coru * dts) * 0.25f, ((cv + wv) + wvn) + cvn, rounded);
+    return (ucor - (zfz * hx) * gzh) - (zcx * zrom1u) * (cp - wp);
   };
   auto eq18 = [&](float cv, float cu, float su, float eu, float esu, float st, float ct, float sp, float cp, float sd0,
                   float sd1, float cd0, float cd1, float corv, float hy, float mv) {
     const float zcy = rot ? dtrdy : dtrdy * mv;
     const float zfz = egdts + 0.25f * (((sd0 + sd1) + cd0) + cd1);
     const float zrom1v = hcpd * (st + ct);
-    const float zcor1v = ((corv * dts) * 0.25f) * (((cu + su) + eu) + esu);
-    return ((cv - zcor1v) - (zfz * hy) * gzh) - (zcy * zrom1v) * (cp - sp);
+    const float vcor = minus_cor(cv, (corv * dts) * 0.25f, ((cu + su) + eu) + esu, rounded);
+    return (vcor - (zfz * hy) * gzh) - (zcy * zrom1v) * (cp - sp);
   };
   if (!in) return;
   const unsigned c = o + r + j0;

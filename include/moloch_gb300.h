@@ -275,6 +275,7 @@ const char* moloch_gpu_kernel_name(int kind);
  *               columns per thread and 16-byte loads and stores (FP32
  *               storage, jx a multiple of 4; elsewhere, and in ensembles,
  *               ignored), 0: one column per thread.
+ * A handle starts with shapes chosen by its size and mode.
  * moloch_gpu_autotune runs advection() and sound() once per candidate and
  * repeat, so it advances the model state: call it on a scratch handle or before the
  * initial state is uploaded again.  The chosen values can be cached by the
