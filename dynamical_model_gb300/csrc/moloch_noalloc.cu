@@ -51,125 +51,297 @@ struct NaArgs {
   int rotllr;
 };
 
-// one vertical pass (:966-1020 / :1022-1072) with inline metric factors
-__device__ void na_vpass(const double* src, double* dst, const NaArgs& a, size_t c) {
-  const size_t pl = (size_t)a.nj * a.ni;
-  const int kz = a.kz;
-  double x0 = src[c], x1 = x0, x2 = src[c + pl];
-  double wfw_k = 0.0, s_k = a.s[c];
-  for (int k = 1; k <= kz; ++k) {
-    const size_t o = (size_t)(k - 1) * pl;
-    const double s_k1 = a.s[c + (size_t)k * pl];
-    const int k2 = k + 2 <= kz ? k + 2 : kz;
-    const double x3 = src[c + (size_t)(k2 - 1) * pl];
-    double wfw_k1 = 0.0;
-    if (k <= kz - 1) {
-      const double zamu = s_k1 * a.dtrdz;
-      double is, num;
-      if (zamu >= 0.0) { is = 1.0; num = x2 - x3; } else { is = -1.0; num = x0 - x1; }
-      const double r = num / safeden(x1 - x2);
-      const double b = superbee(r);
-      const double zphi = (is + zamu * b) - is * b;
-      wfw_k1 = (0.5 * s_k1) * ((1.0 + zphi) * x2 + (1.0 - zphi) * x1);
+// What bounds these kernels: the FP64 pipe (two lanes an SM and clock, 16
+// clocks a warp instruction), not the 9 words of traffic a point.  So every
+// flux, every reciprocal of a metric and every 1 / m of the map factors is
+// computed once and handed on -- down the march, through shared memory or
+// over the levels of a thread -- and comparisons, selects and signs run on
+// the integer pipe.  FP64 instructions a point, both fluxes and every metric
+// factor taken at each point -> now: vertical 112 -> 87, meridional 103 -> 68,
+// zonal 90 -> 51, at 81-87 % of the pipe; one call at 160 x 128 x 64 1060 ->
+// 550 us, 64 x 48 x 30 226 -> 86 us, 200 x 190 x 20 574 -> 349 us, bit for bit
+// the same results.
+
+// 1 / b to half an ulp times 1 + 2^-11.6 (the estimate's third-order step,
+// rounded), and whether na_quot may use it.
+struct NaRcp {
+  double b, y;
+  bool ok;
+};
+__device__ __forceinline__ NaRcp na_rcp(double b) {
+  NaRcp r;
+  r.b = b;
+  r.ok = mid_range(b) && (__double2hiint(b) & 0xffe00) != 0xffe00;
+  const double x = rcp_seed(b), e = __fma_rn(-b, x, 1.0);
+  r.y = __fma_rn(x, __fma_rn(e, e, e), x);
+  return r;
+}
+// a / b, correctly rounded, with Markstein's quotient correction (P.
+// Markstein, "IA-64 and Elementary Functions", 2000): q = a y is within 1.5
+// ulp, the first residual takes it to half an ulp (1 + 2^-49), and the second
+// is exact, so that what is rounded last differs from a / b by at most
+// 2^-107 b (1 + 2^-11.5) where a >= b (a and b scaled to [1, 2)).  A quotient
+// of two doubles is no nearer than 2^-105 / b to the middle of two doubles:
+// the rounding is right while b < 2 (1 - 2^-12.5).  a < b halves both.  Other
+// b, and |a| outside 2^-800 .. 2^800 but 0, divide as IEEE.
+__device__ __forceinline__ double na_quot(double a, const NaRcp& r) {
+  const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  const bool zero = (h | (unsigned)__double2loint(a)) == 0u;
+  if (!(r.ok && (zero || h - 0x0df00000u < 0x71f00000u - 0x0df00000u))) return a / r.b;
+  double q = a * r.y;
+  q = __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
+  return __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
+}
+// 1 / b, correctly rounded (the same with q = y)
+__device__ __forceinline__ double na_inv(double b) {
+  const NaRcp r = na_rcp(b);
+  return r.ok ? __fma_rn(__fma_rn(-b, r.y, 1.0), r.y, r.y) : 1.0 / b;
+}
+// x / 2 by the exponent
+__device__ __forceinline__ double na_half(double x) {
+  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+  if (e - 2u < 0x7ffu - 2u) return __hiloint2double(__double2hiint(x) - 0x100000, __double2loint(x));
+  return 0.5 * x;
+}
+
+// superbee by the bits of r: 0 below 0, 2r up to 1/2, 1 up to 1, r up to 2,
+// then 2; 1 for NaN, as the comparisons of superbee() fall
+__device__ __forceinline__ double na_superbee(double r) {
+  const long long x = __double_as_longlong(r);
+  const long long half = 0x3fe0000000000000LL, one = 0x3ff0000000000000LL, two = 0x4000000000000000LL;
+  long long b = x < one ? one : x;
+  if (x < half) b = x >= 0x0010000000000000LL ? x + 0x0010000000000000LL : x << 1;  // subnormal: twice by a shift
+  if (x >= two) b = two;
+  if (x < 0) b = 0;
+  if ((x & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL) b = one;
+  return __longlong_as_double(b);
+}
+// sign(max(abs(z), minden), z) by the bits of z (NaN becomes minden)
+__device__ __forceinline__ double na_safeden(double z) {
+  const unsigned long long lo = (unsigned long long)__double_as_longlong(kMinden), inf = 0x7ff0000000000000ULL;
+  const unsigned long long x = (unsigned long long)__double_as_longlong(z);
+  unsigned long long m = x & 0x7fffffffffffffffULL;
+  if (m - lo > inf - lo) m = lo;
+  return __longlong_as_double((long long)(m | (x & 0x8000000000000000ULL)));
+}
+
+// (1 + zphi) m1 + (1 - zphi) x0 of the flux between cells m1 and x0; up: the
+// wind comes from m1's side, num the difference that side of it
+__device__ __forceinline__ double na_flux(bool up, double zamu, double num, double den, double m1, double x0) {
+  const double is = up ? 1.0 : -1.0;
+  const double b = na_superbee(na_quot(num, na_rcp(na_safeden(den))));
+  const double zphi = (is + zamu * b) - (up ? b : -b);
+  return (1.0 + zphi) * m1 + (1.0 - zphi) * x0;
+}
+// horizontal flux (:1088-1104); dm, d0, dp: the differences x(i) - x(i-1) at
+// the face before, this one and the next
+__device__ __forceinline__ double na_hflux(double zamu, double dm, double d0, double dp, double m1, double x0) {
+  const bool up = __double_as_longlong(zamu) > 0;
+  return na_flux(up, zamu, up ? dm : dp, d0, m1, x0);
+}
+// flux through the lower face of x1 (:966-1012); d0, d1, d2: x(k) - x(k+1)
+// above x1, below it and below x2
+__device__ __forceinline__ double na_vflux(double s1, double zamu, double d0, double d1, double d2, double x1, double x2) {
+  const long long z = __double_as_longlong(zamu);
+  const bool up = z >= 0 || z == (long long)0x8000000000000000ULL;
+  return na_half(s1) * na_flux(up, zamu, up ? d2 : d0, d1, x2, x1);
+}
+
+// Both vertical passes (:966-1072).  A warp holds 32 columns and up to
+// kNaLevels levels of them, the warps of a block one after the other down the
+// column, so that 1 / fmzf is taken once a face and the metric factors of the
+// first pass stay in registers for the second; what the passes exchange goes
+// through shared memory.  Four to eight levels a warp measure the same within
+// 5 %; two take 12 % more (the first flux of a warp is taken twice).  Columns
+// deeper than kNaWarps kNaLevels march with one thread each
+// (k_na_vertical_deep), which takes every metric factor twice.
+constexpr int kNaLevels = 6, kNaWarps = 12;
+__global__ void __launch_bounds__(32 * kNaWarps) k_na_vertical(NaArgs a) {
+  extern __shared__ double sx[];  // [kz][32]
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const size_t pl = (size_t)a.nj * a.ni, cc = (size_t)blockIdx.x * 32 + lane, c = cc < pl ? cc : pl - 1;
+  const int kz = a.kz, lv = (kz + nw - 1) / nw, k0 = w * lv, k1 = min(k0 + lv, kz);
+  for (int k = k0; k < k1; ++k) sx[k * 32 + lane] = a.pp[c + k * pl];
+  __syncthreads();
+  double zu[kNaLevels], zd[kNaLevels], dv[kNaLevels], xo[kNaLevels];
+  auto X = [&](int k) { return sx[min(max(k, 0), kz - 1) * 32 + lane]; };
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    if (k0 < k1) {
+      NaRcp r0;
+      if (pass == 0) r0 = na_rcp(a.fmzf[c + k0 * pl]);
+      double x1 = X(k0), x2 = X(k0 + 1), d0 = X(k0 - 1) - x1, d1 = x1 - x2;
+      double s0 = a.s[c + k0 * pl], w0 = 0.0;
+      if (k0 > 0) w0 = na_vflux(s0, s0 * a.dtrdz, X(k0 - 2) - X(k0 - 1), d0, d1, X(k0 - 1), x1);
+#pragma unroll
+      for (int n = 0; n < kNaLevels; ++n) {
+        const int k = k0 + n;
+        if (k < k1) {
+          const double s1 = a.s[c + (k + 1) * pl], x3 = X(k + 2), d2 = x2 - x3;
+          const double w1 = k < kz - 1 ? na_vflux(s1, s1 * a.dtrdz, d0, d1, d2, x1, x2) : 0.0;
+          if (pass == 0) {
+            const double f = a.dtrdz * a.fmz[c + k * pl];
+            const NaRcp r1 = na_rcp(a.fmzf[c + (k + 1) * pl]);
+            zu[n] = na_quot(f, r0);
+            zd[n] = na_quot(f, r1);
+            dv[n] = s0 * zu[n] - s1 * zd[n];
+            r0 = r1;
+          }
+          xo[n] = ((x1 - w0 * zu[n]) + w1 * zd[n]) + dv[n] * x1;
+          x1 = x2; x2 = x3; d0 = d1; d1 = d2; w0 = w1; s0 = s1;
+        }
+      }
     }
-    const double f = a.fmz[c + o];
-    const double zrfmu = (a.dtrdz * f) / a.fmzf[c + o];
-    const double zrfmd = (a.dtrdz * f) / a.fmzf[c + o + pl];
-    const double zdv = (s_k * zrfmu - s_k1 * zrfmd) * x1;
-    dst[c + o] = ((x1 - wfw_k * zrfmu) + wfw_k1 * zrfmd) + zdv;
-    x0 = x1; x1 = x2; x2 = x3; wfw_k = wfw_k1; s_k = s_k1;
+    __syncthreads();  // every warp has read what the others overwrite
+#pragma unroll
+    for (int n = 0; n < kNaLevels; ++n)
+      if (k0 + n < k1) {
+        if (pass == 0) sx[(k0 + n) * 32 + lane] = xo[n];
+        else if (cc < pl) a.wz[c + (k0 + n) * pl] = xo[n];
+      }
+    __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(128) k_na_vertical(NaArgs a) {
-  const int jj = blockIdx.x * 32 + threadIdx.x, ii = blockIdx.y * 4 + threadIdx.y;
-  if (jj >= a.nj || ii >= a.ni) return;
-  const size_t c = jj + (size_t)a.nj * ii;
+// one pass down a whole column (:966-1020 / :1022-1072)
+__device__ void na_vpass(const double* src, double* dst, const NaArgs& a, size_t c) {
+  const size_t pl = (size_t)a.nj * a.ni;
+  const int kz = a.kz;
+  double x1 = src[c], x2 = src[c + pl], d0 = 0.0, d1 = x1 - x2;
+  double w0 = 0.0, s0 = a.s[c];
+  NaRcp r0 = na_rcp(a.fmzf[c]);
+  for (int k = 0; k < kz; ++k) {
+    const size_t o = c + k * pl;
+    const double s1 = a.s[o + pl], x3 = src[c + min(k + 2, kz - 1) * pl], d2 = x2 - x3;
+    const double w1 = k < kz - 1 ? na_vflux(s1, s1 * a.dtrdz, d0, d1, d2, x1, x2) : 0.0;
+    const double f = a.dtrdz * a.fmz[o];
+    const NaRcp r1 = na_rcp(a.fmzf[o + pl]);
+    const double zu = na_quot(f, r0), zd = na_quot(f, r1);
+    dst[o] = ((x1 - w0 * zu) + w1 * zd) + (s0 * zu - s1 * zd) * x1;
+    x1 = x2; x2 = x3; d0 = d1; d1 = d2; w0 = w1; s0 = s1; r0 = r1;
+  }
+}
+__global__ void __launch_bounds__(128) k_na_vertical_deep(NaArgs a) {
+  const size_t c = (size_t)blockIdx.x * 128 + threadIdx.x;
+  if (c >= (size_t)a.nj * a.ni) return;
   na_vpass(a.pp, a.wz, a, c);
   na_vpass(a.wz, a.wz, a, c);
 }
 
-// WAF flux between cells m1 and 0 given the neighbours m2 and p1
-__device__ __forceinline__ double na_flux(double zamu, double m2, double m1, double x0, double p1) {
-  double is, num;
-  if (zamu > 0.0) { is = 1.0; num = m1 - m2; } else { is = -1.0; num = p1 - x0; }
-  const double r = num / safeden(x0 - m1);
-  const double b = superbee(r);
-  const double zphi = (is + zamu * b) - is * b;
-  return (1.0 + zphi) * m1 + (1.0 - zphi) * x0;
+// Meridional flux + update (:1080-1131).  A thread marches kNaRows rows of
+// one column: the flux, the reciprocal of fmz(i) + fmz(i+1) and 1 / mv of a
+// face serve both its rows (four rows against 6, 8 and 16: 585, 591, 590 and
+// 611 us a call at 160 x 128 x 64, 84, 82, 87 and 112 at 64 x 48 x 30; two or
+// four levels a thread leave too few warps there, 108 and 157).
+constexpr int kNaRows = 4;
+__global__ void __launch_bounds__(128) k_na_meridional(NaArgs a) {
+  const int nj = a.nj, ni = a.ni, strips = (ni + kNaRows - 1) / kNaRows;
+  const int t = blockIdx.x * 128 + threadIdx.x;
+  if (t >= nj * strips) return;
+  const int jj = t % nj, i0 = (t / nj) * kNaRows, i1 = min(i0 + kNaRows, ni);
+  const size_t pl = (size_t)nj * ni;
+  const size_t ko = blockIdx.y * pl + jj;
+  auto row = [&](int i) { return (size_t)nj * wrap2(i, ni); };
+  auto face = [&](double v, double rm, double dm, double d0, double dp, double m1, double x0) {  // zpby
+    const double vr = a.rotllr ? v : v * rm;
+    const double fl = na_hflux(vr * a.dtrdy, dm, d0, dp, m1, x0);
+    return a.rotllr ? na_half(v) * fl : (na_half(v) * rm) * fl;
+  };
+  double rms = na_inv(a.mv[row(i0) + jj]);
+  const double m2 = a.wz[ko + row(i0 - 2)], m1 = a.wz[ko + row(i0 - 1)];
+  double x1 = a.wz[ko + row(i0)], x2 = a.wz[ko + row(i0 + 1)], d0 = x1 - m1, d1 = x2 - x1;
+  double vs = a.v[ko + row(i0)], fc = a.fmz[ko + row(i0)];
+  double zs = face(vs, rms, m1 - m2, d0, d1, m1, x1);
+  NaRcp rs = na_rcp(fc + a.fmz[ko + row(i0 - 1)]);
+  const double dt2 = a.dtrdy * 2.0;  // (c m) 2 f rounds as ((2 c) m) f
+#pragma unroll 1
+  for (int i = i0; i < i1; ++i) {
+    const size_t rc = row(i), rn = row(i + 1), rnn = row(i + 2);
+    const double rmn = na_inv(a.mv[rn + jj]), mxx = a.mx[rc + jj];
+    const double hn = a.rotllr ? (dt2 * rmn) * mxx : mxx * mxx, hs = a.rotllr ? (dt2 * rms) * mxx : 0.0;
+    const double x3 = a.wz[ko + rnn], vn = a.v[ko + rn], fn = a.fmz[ko + rn], pp = a.pp[ko + rc];
+    const double d2 = x3 - x2, zn = face(vn, rmn, d0, d1, d2, x1, x2);
+    const NaRcp r = na_rcp(fc + fn);
+    double p0;
+    if (a.rotllr) {
+      const double zrfmn = na_quot(hn * fc, r), zrfms = na_quot(hs * fc, rs);
+      const double zdv = (vn * zrfmn - vs * zrfms) * pp;
+      p0 = ((x1 + zs * zrfms) - zn * zrfmn) + zdv;
+    } else {
+      const double h = dt2 * fc;
+      const double zrfmn = na_quot(h, r), zrfms = na_quot(h, rs);
+      const double zdv = ((vn * rmn) * zrfmn - (vs * rms) * zrfms) * pp;
+      p0 = x1 + hn * (((zs * zrfms) - zn * zrfmn) + zdv);
+    }
+    a.p0[ko + rc] = p0;
+    x1 = x2; x2 = x3; d0 = d1; d1 = d2; fc = fn; vs = vn; zs = zn; rs = r;
+    rms = rmn;
+  }
 }
 
-// meridional flux + update (:1080-1131); each point evaluates its two fluxes
-__global__ void __launch_bounds__(256) k_na_meridional(NaArgs a) {
-  const int jj = blockIdx.x * 32 + threadIdx.x, ii = blockIdx.y * 8 + threadIdx.y, kk = blockIdx.z;
-  const int nj = a.nj, ni = a.ni;
-  if (jj >= nj || ii >= ni) return;
-  const size_t ko = (size_t)kk * nj * ni;
-  auto W = [&](int i) { return a.wz[ko + jj + (size_t)nj * wrapn(i, ni)]; };
-  auto V = [&](int i) { return a.v[ko + jj + (size_t)nj * wrapn(i, ni)]; };
-  auto RMV = [&](int i) { return 1.0 / a.mv[jj + (size_t)nj * wrapn(i, ni)]; };
-  double zp[2];
-  for (int n = 0; n < 2; ++n) {  // zpby at i and i+1
-    const int i = ii + n;
-    const double vv = V(i);
-    const double zamu = a.rotllr ? vv * a.dtrdy : (vv * RMV(i)) * a.dtrdy;
-    const double fl = na_flux(zamu, W(i - 2), W(i - 1), W(i), W(i + 1));
-    zp[n] = a.rotllr ? (0.5 * vv) * fl : ((0.5 * vv) * RMV(i)) * fl;
+// Zonal flux + update of pp (:1138-1187).  A thread takes one western face
+// and one point of kNaZonK levels; faces go to the points through shared
+// memory.  A block holds `rows` whole rows of nj points, or one segment of a
+// row (one face more than points) where nj is above kNaSeg.
+constexpr int kNaSeg = 256, kNaZonK = 2;
+__global__ void __launch_bounds__(kNaSeg) k_na_zonal(NaArgs a, int rows, int len, int faces, int segs) {
+  __shared__ double sz[kNaZonK][kNaSeg], sy[kNaZonK][kNaSeg], sb[kNaZonK][kNaSeg], sm[kNaSeg];
+  __shared__ bool sk[kNaZonK][kNaSeg];
+  const int nj = a.nj, ni = a.ni, t = threadIdx.x;
+  const size_t pl = (size_t)nj * ni;
+  const int r = t / faces, jf = t - r * faces;
+  const int ii = (blockIdx.x / segs) * rows + r, j0 = (blockIdx.x % segs) * len;
+  const int jp = j0 + jf;  // nj itself is the face 0 of the next image
+  const bool face = r < rows && ii < ni && jp <= nj;
+  const size_t row = (size_t)nj * ii;
+  const int kk = blockIdx.y * kNaZonK, nk = min(kNaZonK, a.kz - kk);
+  const int jc = wrap2(jp, nj), jm = wm1(jc, nj), jm2 = wm1(jm, nj), je = wp1(jc, nj);
+  double x1[kNaZonK], fc[kNaZonK], uw[kNaZonK];
+  if (face) {
+    const double mu = a.mu[row + jc], m = a.rotllr ? mu : na_inv(mu);
+    sm[t] = m;
+#pragma unroll
+    for (int n = 0; n < kNaZonK; ++n) {
+      const size_t o = (size_t)(kk + min(n, nk - 1)) * pl + row;
+      const double u = a.u[o + jc], xw = a.p0[o + jm];
+      x1[n] = a.p0[o + jc];
+      fc[n] = a.fmz[o + jc];
+      uw[n] = u;
+      const double zamu = (u * m) * a.dtrdx;
+      const bool up = __double_as_longlong(zamu) > 0;
+      const double num = (up ? xw : a.p0[o + je]) - (up ? a.p0[o + jm2] : x1[n]);
+      const double fl = na_flux(up, zamu, num, x1[n] - xw, xw, x1[n]);
+      sz[n][t] = a.rotllr ? na_half(u) * fl : (na_half(u) * m) * fl;
+      const NaRcp y = na_rcp(fc[n] + a.fmz[o + jm]);
+      sb[n][t] = y.b;
+      sy[n][t] = y.y;
+      sk[n][t] = y.ok;
+    }
   }
-  const size_t c = jj + (size_t)nj * ii;
-  const double f = a.fmz[ko + c], fn = a.fmz[ko + jj + (size_t)nj * wrapn(ii + 1, ni)];
-  const double fs = a.fmz[ko + jj + (size_t)nj * wrapn(ii - 1, ni)];
-  const double pp = a.pp[ko + c], vs = V(ii), vn = V(ii + 1);
-  double p0;
-  if (a.rotllr) {
-    const double mxx = a.mx[c];
-    const double zhxvtn = (a.dtrdy * RMV(ii + 1)) * mxx, zhxvts = (a.dtrdy * RMV(ii)) * mxx;
-    const double zrfmn = ((zhxvtn * 2.0) * f) / (f + fn), zrfms = ((zhxvts * 2.0) * f) / (f + fs);
-    const double zdv = (vn * zrfmn - vs * zrfms) * pp;
-    p0 = ((W(ii) + zp[0] * zrfms) - zp[1] * zrfmn) + zdv;
-  } else {
-    const double zrfmn = ((a.dtrdy * 2.0) * f) / (f + fn), zrfms = ((a.dtrdy * 2.0) * f) / (f + fs);
-    const double zdv = ((vn * RMV(ii + 1)) * zrfmn - (vs * RMV(ii)) * zrfms) * pp;
-    const double mx2 = a.mx[c] * a.mx[c];
-    p0 = W(ii) + mx2 * (((zp[0] * zrfms) - zp[1] * zrfmn) + zdv);
+  __syncthreads();
+  if (!face || jf >= len || jp >= nj) return;
+  const int e = (faces == nj && jf == nj - 1) ? t - jf : t + 1;  // the eastern face
+  const double m = sm[t], me = sm[e], mx = a.mx[row + jc], dt2 = a.dtrdx * 2.0;
+#pragma unroll
+  for (int n = 0; n < kNaZonK; ++n) {
+    if (n >= nk) break;
+    const size_t o = (size_t)(kk + n) * pl + row;
+    const double ue = a.u[o + je], pp = a.pp[o + jc];
+    const NaRcp re = {sb[n][e], sy[n][e], sk[n][e]}, rw = {sb[n][t], sy[n][t], sk[n][t]};
+    double out;
+    if (a.rotllr) {
+      const double h = (dt2 * m) * fc[n];
+      const double zrfme = na_quot(h, re), zrfmw = na_quot(h, rw);
+      const double zdv = (ue * zrfme - uw[n] * zrfmw) * pp;
+      out = ((x1[n] + sz[n][t] * zrfmw) - sz[n][e] * zrfme) + zdv;
+    } else {
+      const double h = dt2 * fc[n];
+      const double zrfme = na_quot(h, re), zrfmw = na_quot(h, rw);
+      const double zdv = ((ue * me) * zrfme - (uw[n] * m) * zrfmw) * pp;
+      out = x1[n] + (mx * mx) * (((sz[n][t] * zrfmw) - sz[n][e] * zrfme) + zdv);
+    }
+    a.pp[o + jc] = out;
   }
-  a.p0[ko + c] = p0;
-}
-
-// zonal flux + update of pp (:1138-1187)
-__global__ void __launch_bounds__(256) k_na_zonal(NaArgs a) {
-  const int jj = blockIdx.x * 32 + threadIdx.x, ii = blockIdx.y * 8 + threadIdx.y, kk = blockIdx.z;
-  const int nj = a.nj, ni = a.ni;
-  if (jj >= nj || ii >= ni) return;
-  const size_t ko = (size_t)kk * nj * ni, row = (size_t)nj * ii;
-  auto P = [&](int j) { return a.p0[ko + row + wrapn(j, nj)]; };
-  auto U = [&](int j) { return a.u[ko + row + wrapn(j, nj)]; };
-  auto MU = [&](int j) { return a.mu[row + wrapn(j, nj)]; };
-  double zp[2];
-  for (int n = 0; n < 2; ++n) {  // zpbw at j and j+1
-    const int j = jj + n;
-    const double uu = U(j);
-    const double m = a.rotllr ? MU(j) : 1.0 / MU(j);
-    const double zamu = (uu * m) * a.dtrdx;
-    const double fl = na_flux(zamu, P(j - 2), P(j - 1), P(j), P(j + 1));
-    zp[n] = a.rotllr ? (0.5 * uu) * fl : ((0.5 * uu) * m) * fl;
-  }
-  const size_t c = row + jj;
-  const double f = a.fmz[ko + c], fe = a.fmz[ko + row + wrapn(jj + 1, nj)], fw = a.fmz[ko + row + wrapn(jj - 1, nj)];
-  const double pp = a.pp[ko + c], uw = U(jj), ue = U(jj + 1);
-  double out;
-  if (a.rotllr) {
-    const double zcostx = a.dtrdx * MU(jj);
-    const double zrfme = ((zcostx * 2.0) * f) / (f + fe), zrfmw = ((zcostx * 2.0) * f) / (f + fw);
-    const double zdv = (ue * zrfme - uw * zrfmw) * pp;
-    out = ((P(jj) + zp[0] * zrfmw) - zp[1] * zrfme) + zdv;
-  } else {
-    const double zrfme = ((a.dtrdx * 2.0) * f) / (f + fe), zrfmw = ((a.dtrdx * 2.0) * f) / (f + fw);
-    const double zdv = ((ue * (1.0 / MU(jj + 1))) * zrfme - (uw * (1.0 / MU(jj))) * zrfmw) * pp;
-    const double mx2 = a.mx[c] * a.mx[c];
-    out = P(jj) + mx2 * (((zp[0] * zrfmw) - zp[1] * zrfme) + zdv);
-  }
-  a.pp[ko + c] = out;
 }
 
 // device address of g_scratch, looked up once per device
@@ -243,11 +415,29 @@ extern "C" int moloch_gpu_wafone_noalloc(double* pp, const double* s, const doub
   // each launch's own status: cudaGetLastError here would also return (and
   // clear) an error the caller left pending before this call
   void* args[] = {&a};
-  const dim3 gv((jx + 31) / 32, (iy + 3) / 4), bv(32, 4);
-  const dim3 gh((jx + 31) / 32, (iy + 7) / 8, kz), bh(32, 8);
-  e = cudaLaunchKernel((const void*)k_na_vertical, gv, bv, args, 0, st);
-  if (e == cudaSuccess) e = cudaLaunchKernel((const void*)k_na_meridional, gh, bh, args, 0, st);
-  if (e == cudaSuccess) e = cudaLaunchKernel((const void*)k_na_zonal, gh, bh, args, 0, st);
+  const int pl = jx * iy;
+  // fewest warps that hold the column, at most kNaLevels levels each
+  const int nw = (kz + kNaLevels - 1) / kNaLevels;
+  if (nw <= kNaWarps)
+    e = cudaLaunchKernel((const void*)k_na_vertical, dim3((pl + 31) / 32), dim3(32 * nw), args, (size_t)kz * 32 * 8, st);
+  else
+    e = cudaLaunchKernel((const void*)k_na_vertical_deep, dim3((pl + 127) / 128), dim3(128), args, 0, st);
+  const int strips = (iy + kNaRows - 1) / kNaRows;
+  if (e == cudaSuccess)
+    e = cudaLaunchKernel((const void*)k_na_meridional, dim3((jx * strips + 127) / 128, kz),
+                         dim3(128), args, 0, st);
+  int rows = 1, len = jx, faces = jx, segs = 1;
+  if (jx > kNaSeg) {
+    segs = (jx + kNaSeg - 2) / (kNaSeg - 1);
+    len = (jx + segs - 1) / segs;
+    faces = len + 1;
+  } else {
+    rows = kNaSeg / jx < iy ? kNaSeg / jx : iy;
+  }
+  void* zargs[] = {&a, &rows, &len, &faces, &segs};
+  if (e == cudaSuccess)
+    e = cudaLaunchKernel((const void*)k_na_zonal, dim3((iy + rows - 1) / rows * segs, (kz + kNaZonK - 1) / kNaZonK),
+                         dim3((rows * faces + 31) / 32 * 32), zargs, 0, st);
   if (e != cudaSuccess) {
     moloch_internal_set_error(cudaGetErrorString(e));
     return MOLOCH_ERR_CUDA;
