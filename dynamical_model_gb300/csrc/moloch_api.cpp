@@ -280,10 +280,12 @@ PhaseFlags flags_of(const moloch_handle* h) {
 //   FP32, other jx, 203 x 157 x 45: divergence + damping 34 | 30 (fused strips,
 //     one launch less), momentum 25 | 22; at 64 x 64 x 30 the strips lose (13 |
 //     21, 8 | 9), so they start at 2^20 points
-//   horizontal WAF, tiles | strips of 16 rows: FP32 27 | 29 at 64 x 64 x 30, 52 |
-//     33 at 100 x 100 x 30, 289 | 111 at 256 x 256 x 40; FP64 71 | 123, 193 | 183,
-//     1073 | 1063; strips of 32 rows from 512 x 512 in FP32 (586 | 565 at
-//     512 x 512 x 60) and 256 x 256 in FP64 (1420 | 1395 at 256 x 256 x 60)
+//   horizontal WAF, tiles | strips of 16 rows: FP32 with odd jx 27 | 29 at 64 x
+//     64 x 30, 52 | 33 at 100 x 100 x 30, 289 | 111 at 256 x 256 x 40; with even jx
+//     (column pairs) 15 | 14 at 24 x 20 x 12, 16 | 14 at 48 x 40 x 30, 27 | 16, 52 |
+//     21; FP64 71 | 123, 193 | 183, 1073 | 1063; strips of 32 rows from 512 x 512
+//     in FP32 (453 | 450 at 512 x 512 x 60, 1776 | 1716 at 1024 x 1024 x 60) and
+//     256 x 256 in FP64 (1420 | 1395 at 256 x 256 x 60)
 //   vertical WAF, FP64, fields a thread 1 | 2 | 5: 43 | 45 | 83 at 48 x 40 x 20,
 //     186 | 164 | 178 at 100 x 100 x 30, 660 | 609 | 550 at 203 x 157 x 45
 //   FP64 divergence, damping, momentum, a level a thread | k-marching: 18, 18,
@@ -301,7 +303,7 @@ void default_shapes(View<T>& v, int mode) {
   v.cor_rounded = 1;
   if (mode == MOLOCH_FP32_MIXED) {
     v.srows = 8;
-    if (pts >= 200000) v.hz_levels = cols >= 200000 ? 32 : 16;
+    if (pts >= 200000 || v.nj % 2 == 0) v.hz_levels = cols >= 200000 ? 32 : 16;
     if (v.nj % 4 == 0) {
       v.kmarch = 16 | 512 | 32 | 128 | 8 | 64;
       v.stag4 = 1;

@@ -3382,6 +3382,195 @@ __device__ __forceinline__ void b_waf_hstrip(const View<T>& d, const int bx, con
   }
 }
 
+// FP32 with jx even: strips of 60 output columns, two (j, j+1) per lane.  The
+// one-column strips are bound by issue slots (105 instructions a point, 77 %
+// of the slots); here sums, products and fused operations take both columns
+// in one instruction, of the four p0 neighbours and the next flux a pair needs
+// four shuffles instead of eight, and 60 of 64 columns are output instead of
+// 28 of 32.  Each warp takes five of the ten fields -- ten need 250 registers,
+// 4.83 instead of 5.04 ms at 1024 x 1024 x 60 but 0.339 instead of 0.271 at 256
+// x 256 x 40 -- the groups of a strip run together and share the rows of
+// winds and metric terms in L2, and the next row travels through shared memory
+// (in registers it spills: 5.39 ms).  Three blocks an SM (154 registers): four
+// with 16 bytes spilled 5.68 ms.  Every rounding is that of the one-column
+// form.  Per step, one column -> two: 1024 x 1024 x 60 6.08 -> 5.04 ms, 512 x
+// 512 x 60 1.62 -> 1.35, 256 x 256 x 40 0.381 -> 0.271, 202 x 157 x 45 0.220 ->
+// 0.159, 100 x 100 x 30 0.098 -> 0.060.
+struct HFace2 {
+  bool p0, p1;  // the positive direction is upwind
+  f32x2 nis, zm;  // -is, is - zamu
+};
+__device__ __forceinline__ HFace2 hface2(f32x2 vel, f32x2 dt) {
+  HFace2 f;
+  const f32x2 z = mul2(vel, dt);
+  const float2 zz = unpack2(z);
+  f.p0 = zz.x > 0.f;
+  f.p1 = zz.y > 0.f;
+  f.nis = pack2(f.p0 ? -1.f : 1.f, f.p1 ? -1.f : 1.f);
+  f.zm = sub2(pack2(f.p0 ? 1.f : -1.f, f.p1 ? 1.f : -1.f), z);
+  return f;
+}
+// WAF value between m1 and x0, n0 and n1 the upwind differences, d = x0 - m1
+__device__ __forceinline__ f32x2 hflux2(const HFace2& f, float n0, float n1, f32x2 d, f32x2 m1, f32x2 x0) {
+  const float2 b = unpack2(d);
+  const f32x2 bb = pack2(bb_of(n0, b.x), bb_of(n1, b.y));
+  return fma2(fma2(bb, f.zm, f.nis), d, add2(m1, x0));
+}
+constexpr int kHPairJ = 60;
+constexpr int kHPG = 5, kHPAhead = 1, kHPArrays = 2 * kHPG + 9;  // fields per warp, rows ahead
+constexpr int kHPSmem = (kHPAhead + 1) * kHPArrays * 128 * 8;
+// a b, a product that no sum may absorb (the assembler fuses mul.rn.f32x2
+// with an add.rn.f32x2 that follows it)
+__device__ __forceinline__ f32x2 product2(f32x2 a, f32x2 b) {
+  const float2 x = unpack2(a), y = unpack2(b);
+  return pack2(__fmul_rn(x.x, y.x), __fmul_rn(x.y, y.y));
+}
+template <bool ROT>
+__device__ __forceinline__ void b_waf_hpair(const View<float>& d, const int bx, const int k, const int g0) {
+  constexpr int G = kHPG;
+  static_assert(kNumAdvected % G == 0, "fields per group");
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nj = d.nj, ni = d.ni, kz = d.kz;
+  const unsigned pl = (unsigned)d.pl;
+  const int R = d.hz_levels;
+  const int nsj = (nj + kHPairJ - 1) / kHPairJ, nsi = (ni + R - 1) / R;
+  const int w = bx * (blockDim.x >> 5) + wid;
+  if (w >= nsj * nsi) return;  // whole warp
+  const int sj = w % nsj, si = w / nsj;
+  const int jl = sj * kHPairJ - 2 + 2 * lane;  // this lane's first column before wrapping
+  const int j = wrapn(jl, nj);
+  const bool out_lane = lane >= 1 && lane < 31 && jl < nj;
+  const int i_s = si * R, i_e = min(i_s + R, ni);
+  auto ld = [](const float* q) -> f32x2 { return pack2(*reinterpret_cast<const float2*>(q)); };
+  const float* __restrict__ u = d.ubuf[d.cur] + (size_t)k * pl;
+  const float* __restrict__ v = d.vbuf[d.cur] + (size_t)k * pl;
+  const float* __restrict__ wn_ = d.wafn + (size_t)k * pl;
+  const float* __restrict__ ws_ = d.wafs + (size_t)k * pl;
+  const float* __restrict__ we_ = d.wafe + (size_t)k * pl;
+  const float* __restrict__ ww_ = d.wafw + (size_t)k * pl;
+  const f32x2 dtx = pack2(d.dtrdx_a, d.dtrdx_a), dty = pack2(d.dtrdy_a, d.dtrdy_a);
+  const f32x2 half = pack2(0.5f, 0.5f), neg = pack2(-1.f, -1.f);
+  auto row = [&](int i) { return (unsigned)j + (unsigned)nj * (unsigned)wrap2(i, ni); };
+  {
+    const float* wz[G];
+    const float* pp[G];
+    float* out[G];
+    f32x2 w0[G], w1[G], da[G], db[G], fl[G];  // wz(i), wz(i+1), their differences, the flux of face i
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      wz[g] = d.wz + ((size_t)(g0 + g) * kz + k) * pl;
+      pp[g] = d.fset[d.fcur][g0 + g] + (size_t)k * pl;
+      out[g] = d.fset[d.fcur ^ 1][g0 + g] + (size_t)k * pl;
+    }
+    auto mflux = [&](const HFace2& f, f32x2 dm, f32x2 d0, f32x2 dp, f32x2 m1, f32x2 x0) {
+      const float2 a = unpack2(dm), c = unpack2(dp);
+      return hflux2(f, f.p0 ? a.x : c.x, f.p1 ? a.y : c.y, d0, m1, x0);
+    };
+    f32x2 v_i;  // v at the face below row i (times 1 / msfv, non-ROTLLR)
+    {
+      const unsigned r = row(i_s), r2 = row(i_s - 2), r1 = row(i_s - 1), rp = row(i_s + 1);
+      v_i = ld(v + r);
+      const f32x2 rm = ROT ? neg : ld(d.rmv + r);
+      const f32x2 fac = ROT ? mul2(half, v_i) : mul2(mul2(half, v_i), rm);
+      if (!ROT) v_i = mul2(v_i, rm);
+      const HFace2 f = hface2(v_i, dty);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const f32x2 a = ld(wz[g] + r2), b = ld(wz[g] + r1);
+        w0[g] = ld(wz[g] + r);
+        w1[g] = ld(wz[g] + rp);
+        da[g] = sub2(w0[g], b);
+        db[g] = sub2(w1[g], w0[g]);
+        fl[g] = mul2(fac, mflux(f, sub2(b, a), da[g], db[g], b, w0[g]));
+      }
+    }
+    // row i's values travel kHPAhead rows ahead through the thread's own
+    // slots of shared memory
+    extern __shared__ float2 hp_ring[];
+    float2* const slot0 = hp_ring + threadIdx.x;
+    auto fetch_row = [&](int i, int st) {
+      if (i < i_e) {
+        float2* q = slot0 + st * (kHPArrays * 128);
+        const unsigned r = row(i), rn = row(i + 1), r2 = row(i + 2);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          cp_async8(q + g * 128, wz[g] + r2);
+          cp_async8(q + (G + g) * 128, pp[g] + r);
+        }
+        q += 2 * G * 128;
+        cp_async8(q, v + rn);
+        cp_async8(q + 128, wn_ + r);
+        cp_async8(q + 2 * 128, ws_ + r);
+        cp_async8(q + 3 * 128, u + r);
+        cp_async8(q + 4 * 128, we_ + r);
+        cp_async8(q + 5 * 128, ww_ + r);
+        cp_async8(q + 6 * 128, (ROT ? d.mu : d.rmu) + r);
+        if (!ROT) {
+          cp_async8(q + 7 * 128, d.rmv + rn);
+          cp_async8(q + 8 * 128, d.mx2 + r);
+        }
+      }
+      cp_async_commit();
+    };
+#pragma unroll
+    for (int n = 0; n < kHPAhead; ++n) fetch_row(i_s + n, n);
+    int rd = 0;
+#pragma unroll 1
+    for (int i = i_s; i < i_e; ++i) {
+      const unsigned r = row(i);
+      cp_async_wait<kHPAhead - 1>();
+      const float2* q = slot0 + rd * (kHPArrays * 128);
+      const float2* qs = q + 2 * G * 128;
+      const f32x2 vr = pack2(qs[0]), pn = pack2(qs[128]), ps = pack2(qs[2 * 128]), uu = pack2(qs[3 * 128]), oe = pack2(qs[4 * 128]),
+                  ow = pack2(qs[5 * 128]), zmf = pack2(qs[6 * 128]);
+      const f32x2 rmv = ROT ? neg : pack2(qs[7 * 128]), mx2 = ROT ? neg : pack2(qs[8 * 128]);
+      const f32x2 uz = mul2(uu, zmf);
+      const f32x2 v_n = ROT ? vr : mul2(vr, rmv), uf = ROT ? uu : uz;
+      const f32x2 mfac = ROT ? mul2(half, vr) : mul2(mul2(half, vr), rmv);
+      const f32x2 zfac = ROT ? mul2(half, uu) : mul2(mul2(half, uu), zmf);
+      const HFace2 fm = hface2(v_n, dty), fz = hface2(uz, dtx);
+      const float2 ufx = unpack2(uf);
+      const f32x2 ufe = pack2(ufx.y, __shfl_down_sync(0xffffffffu, ufx.x, 1));
+      const f32x2 npn = mul2(pn, neg), noe = mul2(oe, neg);
+      // a b - c d: the first product is fused, as in the one-column form
+      const f32x2 pdv = fma2(v_n, pn, mul2(v_i, mul2(ps, neg)));
+      const f32x2 odv = fma2(ufe, oe, mul2(uf, mul2(ow, neg)));
+      f32x2 wp2[G], pold[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g) { wp2[g] = pack2(q[g * 128]); pold[g] = pack2(q[(G + g) * 128]); }
+      fetch_row(i + kHPAhead, rd == 0 ? kHPAhead : rd - 1);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const f32x2 dn = sub2(wp2[g], w1[g]);
+        const f32x2 fn = mul2(mfac, mflux(fm, da[g], db[g], dn, w0[g], w1[g]));  // face i+1
+        const f32x2 p0 = ROT ? fma2(pdv, pold[g], fma2(fn, npn, fma2(fl[g], ps, w0[g])))
+                             : fma2(mx2, fma2(pdv, pold[g], fma2(fl[g], ps, mul2(fn, npn))), w0[g]);
+        w0[g] = w1[g]; w1[g] = wp2[g]; da[g] = db[g]; db[g] = dn; fl[g] = fn;
+        const float2 p = unpack2(p0);
+        const float pm2 = __shfl_up_sync(0xffffffffu, p.x, 1), pm1 = __shfl_up_sync(0xffffffffu, p.y, 1);
+        const float pp1 = __shfl_down_sync(0xffffffffu, p.x, 1);
+        const f32x2 m1 = pack2(pm1, p.x), dz = sub2(p0, m1);
+        const float2 z = unpack2(dz), e = unpack2(sub2(pack2(pm1, pp1), pack2(pm2, p.y)));
+        const f32x2 zf = mul2(zfac, hflux2(fz, fz.p0 ? e.x : z.y, fz.p1 ? z.x : e.y, dz, m1, p0));  // western faces
+        const float2 zz = unpack2(zf);
+        const f32x2 zfe = pack2(zz.y, __shfl_down_sync(0xffffffffu, zz.x, 1));
+        const f32x2 zdv = product2(odv, pold[g]);  // not fused, as in the one-column form
+        const f32x2 o = ROT ? add2(zdv, fma2(zfe, noe, fma2(zf, ow, p0)))
+                            : fma2(mx2, add2(zdv, fma2(zf, ow, mul2(zfe, noe))), p0);
+        if (out_lane) *reinterpret_cast<float2*>(out[g] + r) = unpack2(o);
+      }
+      v_i = v_n;
+      rd = rd == kHPAhead ? 0 : rd + 1;
+    }
+    cp_async_wait<0>();
+  }
+}
+template <bool ROT>
+__global__ void __launch_bounds__(128, 3) k_waf_hpair(View<float> d) {
+  constexpr int NG = kNumAdvected / kHPG;
+  b_waf_hpair<ROT>(d, blockIdx.x / NG, blockIdx.y, (blockIdx.x % NG) * kHPG);
+}
+
 template <class T>
 __global__ void __launch_bounds__(128) k_waf_hstrip(View<T> d) {
   b_waf_hstrip<T>(d, blockIdx.x, blockIdx.y);
@@ -3838,7 +4027,18 @@ int launch_advection(View<T>& d, cudaStream_t st) {
   const dim3 pb(kPtBX, kPtBY), pg = pt_grid(d.nj, d.ni, d.kz);
   const dim3 hg((d.nj + 31) / 32, (d.ni + 7) / 8, (d.kz + d.hz_levels - 1) / d.hz_levels);
   launch_waf_vertical<T>(d, st);  // forms ux, vx, wx from u, v, w as well
-  if (d.hz_levels >= 16) {  // warp strips of hz_levels rows
+  bool pairs = false;  // jx even: 8-byte loads of column pairs; faster at every size
+  if constexpr (sizeof(T) == 4) {
+    pairs = d.hz_levels >= 16 && d.nj % 2 == 0;
+    if (pairs) {
+      const int np = ((d.nj + kHPairJ - 1) / kHPairJ) * ((d.ni + d.hz_levels - 1) / d.hz_levels);
+      const dim3 g((np + 3) / 4 * (kNumAdvected / kHPG), d.kz);
+      if (d.rotllr) MOLOCH_LAUNCH(KK_WAF_HORIZONTAL, st, k_waf_hpair<true><<<g, 128, kHPSmem, st>>>(d));
+      else MOLOCH_LAUNCH(KK_WAF_HORIZONTAL, st, k_waf_hpair<false><<<g, 128, kHPSmem, st>>>(d));
+    }
+  }
+  if (pairs) {
+  } else if (d.hz_levels >= 16) {  // warp strips of hz_levels rows
     const int nstrips = ((d.nj + kStripJ - 1) / kStripJ) * ((d.ni + d.hz_levels - 1) / d.hz_levels);
     MOLOCH_LAUNCH(KK_WAF_HORIZONTAL, st, k_waf_hstrip<T><<<dim3((nstrips + 3) / 4, d.kz), 128, 0, st>>>(d));
   } else {
