@@ -23,6 +23,7 @@
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <type_traits>
 
@@ -858,6 +859,159 @@ __global__ void __launch_bounds__(kColBX* kColBY, sizeof(T) == 4 && PD == 1 ? 9 
     k_sound_column(View<T> d, int nsound, int last, int defer_pai) {
   b_sound_column<T, PD>(d, blockIdx.x * kColBX + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, nsound, last,
                         defer_pai);
+}
+
+// FP64 on few columns: a block holds C columns (C neighbours of the plane,
+// across row ends) and all their levels.  Its 256 threads form the
+// right-hand sides and coefficients of all levels side by side, C of them run
+// the recurrence down and the substitution up through shared memory, then all
+// of them update Exner function, theta and pai.  Same expressions as the
+// march.
+constexpr int kSplitThreads = 256;
+constexpr size_t split_smem_bytes(int columns, int kz) { return (size_t)3 * kz * columns * sizeof(double); }
+template <int C>
+__global__ void __launch_bounds__(kSplitThreads, 4)
+    k_sound_column_split(View<double> d, int nsound, int last, int defer_pai) {
+  if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
+  extern __shared__ double split_smem[];
+  constexpr int NG = kSplitThreads / C;
+  const int kz = d.kz, nj = d.nj, ni = d.ni;
+  const size_t pl = d.pl;
+  double* const sx = split_smem;  // [level][column]: right-hand side, then wp, then w
+  double* const su = sx + kz * C;  // zu, then wwkw
+  double* const sd = su + kz * C;  // zd
+  const int col = threadIdx.x % C, grp = threadIdx.x / C;
+  const size_t cc = (size_t)blockIdx.x * C + col;
+  const bool on = cc < pl;
+  const size_t c = on ? cc : pl - 1;
+  double* __restrict__ W = d.w + c;
+  const double* __restrict__ FMZF = d.fmzf + c;
+  const double* __restrict__ FMZ = d.fmz + c;
+  const double* __restrict__ QV = d.q[0] + c;
+  const double* __restrict__ QC = d.q[1] + c;
+  double* __restrict__ TET = d.tetav + c;
+  double* __restrict__ PAI = d.pai + c;
+  const double* __restrict__ QSAT = d.qsat + c;
+  const double* __restrict__ TT = d.t + c;
+  double* __restrict__ ZD = d.zdiv2b + c;
+  const double* __restrict__ QWL = d.qwltot + c;
+  const double* __restrict__ QWI = d.qwitot + c;
+  double* __restrict__ S = d.s + c;
+  double* __restrict__ DW = d.deltaw + c;
+  const double dts = d.dts, egdts = d.egdts, dtrdz = d.dtrdz, zcs2 = d.zcs2;
+  const double ns = nsound, ns1 = nsound - 1;
+  const double c2 = 2.0 * ns * dtrdz;
+  const double* __restrict__ FZD = kLean<double> ? d.fzd + c : FMZ;
+  const double wsurf = W[(size_t)kz * pl];
+
+  // coefficients of levels kz .. 2
+  for (int kk = 1 + grp; kk < kz; kk += NG) {
+    const size_t o = (size_t)kk * pl, om = o - pl;
+    const double wk = W[o], fz = FMZF[o], tk = TET[o], tkm = TET[om], pk = PAI[o], pkm = PAI[om];
+    const double zk = ZD[o], zkm = ZD[om], fk = FZD[o], fkm = FZD[om];
+    double ex, zu, zd;
+    if constexpr (kLean<double>) {
+      double zr = mul_rn(mul_rn(0.5 * kCpd, fz), fma_rn(-mul_rn(mul_rn(fz, wk), c2), sub_rn(tkm, tk), add_rn(tkm, tk)));
+      if (__double_as_longlong(wk) > __double_as_longlong(0.1)) {  // latent heat of saturated rising air (:641-652)
+        const double qsk = QSAT[o], qskm = QSAT[om], tm = TT[om];
+        if (QV[o] > 0.96 * qsk) {
+          const double zqs = 0.5 * (qsk + qskm);
+          const double zdth = ((((((kEgrav * wk) * ns1) * dts) * kWlhv) * kWlhv) * zqs) /
+                              ((((kCpd * pkm) * kRwat) * tm) * tm);
+          zr = zr + zdth * fz;
+        }
+      }
+      const double A = mul_rn(zr, dtrdz), B = mul_rn(kRdrcv, A);
+      ex = fma_rn(B, sub_rn(mul_rn(pkm, zkm), mul_rn(pk, zk)), sub_rn(fma_rn(-A, sub_rn(pkm, pk), wk), egdts));
+      zu = mul_rn(B, mul_rn(fkm, pkm));
+      zd = mul_rn(B, mul_rn(fk, pk));
+    } else {
+      double zrom1w = ((0.5 * kCpd) * fz) * (tkm + tk);
+      zrom1w = zrom1w - (((((kCpd * wk) * fz) * fz) * ns) * dtrdz) * (tkm - tk);
+      zrom1w = zrom1w_moist(zrom1w, QV[o], QSAT[o], QSAT[om], wk, fz, pkm, TT[om], ns1, dts);
+      ex = (wk - (zrom1w * dtrdz) * (pkm - pk)) - egdts;
+      ex = ex + ((kRdrcv * zrom1w) * dtrdz) * prod_sub(pkm, zkm, pk, zk);
+      zu = ((zcs2 * fkm) * zrom1w) * pkm + d.ffilt[kk];
+      zd = ((zcs2 * fk) * zrom1w) * pk + d.ffilt[kk];
+    }
+    sx[kk * C + col] = ex;
+    su[kk * C + col] = zu;
+    sd[kk * C + col] = zd;
+  }
+  __syncthreads();
+  if (threadIdx.x < C) {
+    double wkp1 = wsurf, wwp1 = 0.0, cwp1 = 1.0;
+    for (int kk = kz - 1; kk >= 1; --kk) {
+      const double ex = sx[kk * C + col], zu = su[kk * C + col], zd = sd[kk * C + col];
+      if constexpr (kLean<double>) {
+        const double tt = fma_rn(zd, cwp1, 1.0), r = rcp_nr(add_rn(tt, zu));
+        wkp1 = mul_rn(r, fma_rn(zd, wkp1, ex));
+        cwp1 = mul_rn(r, tt);
+        wwp1 = mul_rn(r, zu);
+      } else {
+        const double den = ((1.0 + zd) + zu) - zd * wwp1;
+        const double zrapp = 1.0 / den;
+        wwp1 = zrapp * zu;
+        wkp1 = zrapp * (ex + zd * wkp1);
+      }
+      sx[kk * C + col] = wkp1;
+      su[kk * C + col] = wwp1;
+    }
+    double wl = 0.0;  // w(1) = 0 always (init_moloch :260-262)
+    sx[col] = wl;
+    for (int kk = 1; kk < kz; ++kk) {
+      if constexpr (kLean<double>) wl = fma_rn(su[kk * C + col], wl, sx[kk * C + col]);
+      else wl = sx[kk * C + col] + su[kk * C + col] * wl;
+      sx[kk * C + col] = wl;
+    }
+  }
+  __syncthreads();
+  if (!on) return;
+  // w, deltaw and the Exner/theta update (:690-728)
+  const int jj = (int)(c % nj), ii = (int)(c / nj);
+  for (int m = grp; m < kz; m += NG) {
+    const size_t q = (size_t)m * pl;
+    const double wl = sx[m * C + col], wh = m + 1 < kz ? sx[(m + 1) * C + col] : wsurf;
+    if (m > 0) {
+      DW[q] = kLean<double> ? sub_rn(wl, W[q]) : (-W[q]) + wl;
+      W[q] = wl;
+    }
+    const double tet = TET[q], pai = PAI[q];
+    double zd, r;
+    if constexpr (kLean<double>) {
+      double m1, m2;
+      if (nsound == 1) {
+        const double qv = QV[q], qc = QC[q];
+        m1 = div_nr(fma(3.2, qc, fma(0.86, qv, 1.0)), fma(4.8, qc, fma(0.96, qv, 1.0)));
+        m2 = fma(2.1, QWI[q], fma(4.2, QWL[q], 0.25 * qv));
+        d.mo1[c + q] = m1;
+        d.mo2[c + q] = m2;
+      } else {
+        m1 = d.mo1[c + q];
+        m2 = d.mo2[c + q];
+      }
+      zd = mul_rn(fma_rn(FZD[q], sub_rn(wl, wh), ZD[q]), m1);
+      r = mul_rn(kRdrcv, zd);
+      TET[q] = mul_rn(tet, fma_rn(r, m2, 1.0));  // rounds as the reference's products do
+    } else {
+      const double qv = QV[q], qc = QC[q];
+      zd = ZD[q] + (dtrdz * FMZ[q]) * (wl - wh);
+      zd = div_corr(zd * ((1.0 + 0.86 * qv) + 3.2 * qc), (1.0 + 0.96 * qv) + 4.8 * qc);
+      r = kRdrcv * zd;
+      TET[q] = tet * (1.0 + r * (prod_add(0.25, qv, 4.2, QWL[q]) + 2.1 * QWI[q]));
+    }
+    if (defer_pai) {
+      ZD[q] = zd;
+    } else {
+      if (jj == nj - 1) d.ep_j[ii + (size_t)ni * m] = pai;
+      if (ii == ni - 1) d.ep_i[jj + (size_t)nj * m] = pai;
+      PAI[q] = kLean<double> ? mul_rn(pai, sub_rn(1.0, r)) : pai * (1.0 - r);
+    }
+    if (last) {  // complete Equation 10 (:843-849)
+      S[q] = m == 0 ? 0.0 : kLean<double> ? mul_rn(add_rn(wl, S[q]), FMZF[q]) : (wl + S[q]) * FMZF[q];
+      if (m == kz - 1) S[q + pl] = 0.0;
+    }
+  }
 }
 
 template <class T>
@@ -2359,11 +2513,17 @@ __global__ void __launch_bounds__(kDQThreads, 1) k_divdamp_quad(const __grid_con
   }
 }
 
-inline bool dq_attributes() {
-  cudaFuncSetAttribute(k_divdamp_quad<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_smem_bytes(kDQMaxKz));
-  cudaFuncSetAttribute(k_divdamp_quad<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_smem_bytes(kDQMaxKz));
-  cudaFuncSetAttribute(k_divdamp_quad<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_smem_bytes(kDQMaxKz));
-  return cudaFuncSetAttribute(k_divdamp_quad<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_smem_bytes(kDQMaxKz)) == cudaSuccess;
+// once a device: the attribute is a device's own
+inline void dq_attributes() {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || done[dev].load(std::memory_order_acquire)) return;
+  const int bytes = dq_smem_bytes(kDQMaxKz);
+  cudaFuncSetAttribute(k_divdamp_quad<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaFuncSetAttribute(k_divdamp_quad<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaFuncSetAttribute(k_divdamp_quad<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaFuncSetAttribute(k_divdamp_quad<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  done[dev].store(true, std::memory_order_release);
 }
 
 // ---- advection: vertical WAF, two passes at dt/2 (:966-1073) ------------
@@ -3857,6 +4017,24 @@ inline int sm_count() {
 // the one-thread column solve (variants: k_sound_column)
 template <class T>
 void launch_sound_column(const View<T>& d, cudaStream_t st, int ns, int last, int defer_pai) {
+  if constexpr (sizeof(T) == 8) {
+    // FP64 columns split over a block (k_sound_column_split) while the march
+    // leaves SMs idle.  us per launch, march | 32 columns a block | 8:
+    //   lean   35 | 17 | 14 at 24 x 20 x 12, 55 | 25 | 22 at 53 x 47 x 21, 74 | 33 | 32
+    //          at 64 x 64 x 30, 79 | 50 | 72 at 100 x 100 x 30, 163 | 148 | 250 at
+    //          203 x 157 x 45, 365 | 372 | 659 at 256 x 256 x 60
+    //   exact  47 | 23 | 16, 74 | 34 | 31, 104 | 46 | 47, 104 | 82 | 106; 170 | 178 |
+    //          240 at 150 x 140 x 40
+    // Deeper columns take fewer to a block (48 KB of shared memory).
+    const auto split = [&](auto k, int cols) {
+      MOLOCH_LAUNCH(KK_SOUND_COLUMN, st,
+                    k<<<((unsigned)d.pl + cols - 1) / cols, kSplitThreads, split_smem_bytes(cols, d.kz), st>>>(d, ns, last,
+                                                                                                            defer_pai));
+    };
+    if (d.pl <= 3000 && d.kz <= 256) return split(k_sound_column_split<8>, 8);
+    if (d.pl <= (kLean<T> ? 40000 : 16000) && d.kz <= 64) return split(k_sound_column_split<32>, 32);
+    if (d.pl <= 16000 && d.kz <= 128) return split(k_sound_column_split<16>, 16);
+  }
   const int bj = (d.nj + kColBX - 1) / kColBX;
   const int rows = bj * ((d.ni + kColBY - 1) / kColBY) < 2 * sm_count() ? 1 : kColBY;
   const dim3 cb(kColBX, rows), cg(bj, (d.ni + rows - 1) / rows);
@@ -3902,8 +4080,7 @@ int launch_sound(View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
           if ((d.kmarch & 512) && d.nj % 4 == 0 && d.kz <= kDQMaxKz) {  // four columns per thread
             const int g4 = sm_count(), sm4 = dq_smem_bytes(d.kz);
             const dim3 b4(32, kDQRows + 3);
-            static const bool attr = dq_attributes();
-            (void)attr;
+            dq_attributes();
             if (d.rotllr && last)
               MOLOCH_LAUNCH(KK_SOUND_DIVDAMP, st, k_divdamp_quad<true, 1><<<g4, b4, sm4, st>>>(d));
             else if (d.rotllr)

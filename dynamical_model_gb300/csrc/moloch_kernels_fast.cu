@@ -77,13 +77,11 @@ bool build_column_maps(const View<float>& v, void* out) {
   if (v.kz > kTwMaxKz || v.kz < 2 || v.nj % 4 != 0 || ((uintptr_t)out & 63)) return false;
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return false;
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    cudaFuncSetAttribute(k_sound_column_tw<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<0>::smem);
-    cudaFuncSetAttribute(k_sound_column_tw<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<1>::smem);
-    cudaFuncSetAttribute(kb_sound_column_tw<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<0>::smem);
-    cudaFuncSetAttribute(kb_sound_column_tw<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<1>::smem);
-  });
+  // for the handle's device: the attribute is a device's own
+  cudaFuncSetAttribute(k_sound_column_tw<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<0>::smem);
+  cudaFuncSetAttribute(k_sound_column_tw<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<1>::smem);
+  cudaFuncSetAttribute(kb_sound_column_tw<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<0>::smem);
+  cudaFuncSetAttribute(kb_sound_column_tw<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TwCfg<1>::smem);
   ColumnMaps* cm = static_cast<ColumnMaps*>(out);
   const int nj = v.nj, ni = v.ni, kz = v.kz;
   const int cols = 32 * v.twide, rows = kTwWarps / v.twide, lev = TwCfg<0>::kct;
