@@ -78,6 +78,36 @@ __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, 
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+// Point of a thread in the plane: tile (bx, by) of BX x BY points or, by < 0,
+// the bx-th BX BY points of the plane in order.  FP64 kernels take the plane
+// in order where whole warps a row leave a tenth of the lanes idle: they are
+// bound by the FP64 pipe, whose 16 clocks a warp instruction do not shrink
+// with idle lanes (a row of 100 columns is four warps instead of 3.1).  Per
+// step, rows | in order: 100 x 100 x 30 vertical WAF 0.492 | 0.382 ms, momentum
+// 0.499 | 0.407, divergence 0.284 | 0.249, damping 0.283 | 0.240; 203 x 157 x 45
+// momentum 1.61 | 1.44.  Not worth it where rows fill (150 x 140 x 40, 6 % idle:
+// divergence 0.466 | 0.488) or launches bound (24 x 20 x 12: 0.112 | 0.119).
+template <int BX, int BY, class T>
+__device__ __forceinline__ void point_at(const View<T>& d, const int bx, const int by, int& jj, int& ii) {
+  if (sizeof(T) == 8 && by < 0) {
+    const unsigned q = bx * (BX * BY) + threadIdx.y * BX + threadIdx.x;
+    ii = q / (unsigned)d.nj;
+    jj = q - ii * d.nj;
+  } else {
+    jj = bx * BX + threadIdx.x;
+    ii = by * BY + threadIdx.y;
+  }
+}
+template <class T>
+__host__ __device__ __forceinline__ bool in_order(const View<T>& d) {
+  const int padded = (d.nj + 31) / 32 * 32;
+  return sizeof(T) == 8 && d.pl >= 4096 && 10 * padded >= 11 * d.nj;
+}
+template <class T>
+__device__ __forceinline__ int tile_y(const View<T>& d) {
+  return in_order(d) ? -1 : (int)blockIdx.y;
+}
+
 // Two FP32 values in one 64-bit register pair: sm_103a adds, multiplies and
 // fuses both in one instruction, each rounded as alone.
 typedef unsigned long long f32x2;
@@ -275,8 +305,8 @@ __device__ __forceinline__ T pfwsat(T t, T p) {
 // ---- pre-diagnostics (:289-323) ----------------------------------------
 template <class T>
 __device__ __forceinline__ void b_prediag(const View<T>& d, const int bx, const int by, const int bz, int filterpai, int filtertheta) {
-  int jj = bx * kPtBX + threadIdx.x;
-  int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   if (jj >= d.nj || ii >= d.ni) return;
   size_t c = (size_t)jj + (size_t)d.nj * ii + (size_t)bz * d.pl;
   T pai = d.pai[c], t = d.t[c];
@@ -296,7 +326,7 @@ __device__ __forceinline__ void b_prediag(const View<T>& d, const int bx, const 
 
 template <class T>
 __global__ void __launch_bounds__(kPtBX* kPtBY) k_prediag(View<T> d, int filterpai, int filtertheta) {
-  b_prediag<T>(d, blockIdx.x, blockIdx.y, blockIdx.z, filterpai, filtertheta);
+  b_prediag<T>(d, blockIdx.x, tile_y(d), blockIdx.z, filterpai, filtertheta);
 }
 
 template <class T>
@@ -317,8 +347,8 @@ __global__ void __launch_bounds__(kPtBX* kPtBY)
 template <class T>
 __device__ __forceinline__ void b_sound_div(const View<T>& d, const int bx, const int by, const int bz) {
   if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
-  const int jj = bx * kPtBX + threadIdx.x;
-  const int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int kk = bz;
   const int nj = d.nj, ni = d.ni, kz = d.kz;
   if (jj >= nj || ii >= ni) return;
@@ -384,7 +414,7 @@ __device__ __forceinline__ void b_sound_div(const View<T>& d, const int bx, cons
 
 template <class T>
 __global__ void __launch_bounds__(kPtBX* kPtBY) k_sound_div(View<T> d) {
-  b_sound_div<T>(d, blockIdx.x, blockIdx.y, blockIdx.z);
+  b_sound_div<T>(d, blockIdx.x, tile_y(d), blockIdx.z);
 }
 
 template <class T>
@@ -414,8 +444,8 @@ __device__ __forceinline__ T damp_lean(T ddamp2, T zc, T zw, T ze, T zs, T zn, T
 template <class T>
 __device__ __forceinline__ void b_sound_damp(const View<T>& d, const int bx, const int by, const int bz) {
   if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
-  const int jj = bx * kPtBX + threadIdx.x;
-  const int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int kk = bz;
   const int nj = d.nj, ni = d.ni;
   if (jj >= nj || ii >= ni) return;
@@ -447,7 +477,7 @@ __device__ __forceinline__ void b_sound_damp(const View<T>& d, const int bx, con
 
 template <class T>
 __global__ void __launch_bounds__(kPtBX* kPtBY) k_sound_damp(View<T> d) {
-  b_sound_damp<T>(d, blockIdx.x, blockIdx.y, blockIdx.z);
+  b_sound_damp<T>(d, blockIdx.x, tile_y(d), blockIdx.z);
 }
 
 template <class T>
@@ -1041,8 +1071,8 @@ __device__ __forceinline__ void b_lap_filter(const View<T>& d, const int bx, con
   const T* __restrict__ a = d.zdiv2b;
   T* __restrict__ out = d.zdiv2a;
 
-  int jj = bx * kPtBX + threadIdx.x;
-  int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int nj = d.nj, ni = d.ni;
   if (jj >= nj || ii >= ni) return;
   const size_t o = (size_t)bz * d.pl;
@@ -1057,7 +1087,7 @@ __device__ __forceinline__ void b_lap_filter(const View<T>& d, const int bx, con
 
 template <class T>
 __global__ void __launch_bounds__(kPtBX* kPtBY) k_lap_filter(View<T> d) {
-  b_lap_filter<T>(d, blockIdx.x, blockIdx.y, blockIdx.z);
+  b_lap_filter<T>(d, blockIdx.x, tile_y(d), blockIdx.z);
 }
 
 template <class T>
@@ -1077,8 +1107,8 @@ __device__ __forceinline__ void b_pai_update(const View<T>& d, const int bx, con
   if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
   const T* __restrict__ zd = d.zdiv2a;
 
-  int jj = bx * kPtBX + threadIdx.x;
-  int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int nj = d.nj, ni = d.ni, kk = bz;
   if (jj >= nj || ii >= ni) return;
   const size_t c = jj + (size_t)nj * ii + (size_t)kk * d.pl;
@@ -1090,7 +1120,7 @@ __device__ __forceinline__ void b_pai_update(const View<T>& d, const int bx, con
 
 template <class T>
 __global__ void __launch_bounds__(kPtBX* kPtBY) k_pai_update(View<T> d) {
-  b_pai_update<T>(d, blockIdx.x, blockIdx.y, blockIdx.z);
+  b_pai_update<T>(d, blockIdx.x, tile_y(d), blockIdx.z);
 }
 
 template <class T>
@@ -1111,8 +1141,8 @@ __device__ __forceinline__ void b_filter_increment(const View<T>& d, const int b
   const T* __restrict__ ref = which ? d.tf : d.pf;
   T* __restrict__ out = d.fscr;
 
-  int jj = bx * kPtBX + threadIdx.x;
-  int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int nj = d.nj, ni = d.ni;
   if (jj >= nj || ii >= ni) return;
   const size_t o = (size_t)bz * d.pl;
@@ -1129,7 +1159,7 @@ __device__ __forceinline__ void b_filter_increment(const View<T>& d, const int b
 
 template <class T>
 __global__ void __launch_bounds__(kPtBX* kPtBY) k_filter_increment(View<T> d, int which) {
-  b_filter_increment<T>(d, blockIdx.x, blockIdx.y, blockIdx.z, which);
+  b_filter_increment<T>(d, blockIdx.x, tile_y(d), blockIdx.z, which);
 }
 
 template <class T>
@@ -1160,8 +1190,8 @@ __device__ __forceinline__ T minus_cor(T v, T k, T sum, int rounded) { return pl
 template <class T>
 __device__ __forceinline__ void b_sound_momentum(const View<T>& d, const int bx, const int by, const int bz) {
   if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
-  const int jj = bx * kPtBX + threadIdx.x;
-  const int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int kk = bz;
   const int nj = d.nj, ni = d.ni;
   if (jj >= nj || ii >= ni) return;
@@ -1212,7 +1242,7 @@ __device__ __forceinline__ void b_sound_momentum(const View<T>& d, const int bx,
 
 template <class T>
 __global__ void __launch_bounds__(kPtBX* kPtBY) k_sound_momentum(View<T> d) {
-  b_sound_momentum<T>(d, blockIdx.x, blockIdx.y, blockIdx.z);
+  b_sound_momentum<T>(d, blockIdx.x, tile_y(d), blockIdx.z);
 }
 
 template <class T>
@@ -1234,8 +1264,8 @@ __global__ void __launch_bounds__(kPtBX* kPtBY)
 template <class T>
 __device__ __forceinline__ void b_sound_div_km(const View<T>& d, const int bx, const int by, const int bz) {
   if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
-  const int jj = bx * kPtBX + threadIdx.x;
-  const int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int nj = d.nj, ni = d.ni, kz = d.kz;
   if (jj >= nj || ii >= ni) return;
   const int k0 = bz * kKC, k1 = min(kz, k0 + kKC);
@@ -1321,8 +1351,8 @@ __device__ __forceinline__ void b_sound_div_km(const View<T>& d, const int bx, c
 template <class T>
 __device__ __forceinline__ void b_sound_damp_km(const View<T>& d, const int bx, const int by, const int bz) {
   if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
-  const int jj = bx * kPtBX + threadIdx.x;
-  const int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int nj = d.nj, ni = d.ni;
   if (jj >= nj || ii >= ni) return;
   const int k0 = bz * kKC, k1 = min(d.kz, k0 + kKC);
@@ -1374,8 +1404,8 @@ __device__ __forceinline__ void b_sound_damp_km(const View<T>& d, const int bx, 
 template <class T>
 __device__ __forceinline__ void b_sound_momentum_km(const View<T>& d, const int bx, const int by, const int bz) {
   if (d.sur_skip && *d.sur_skip) return;  // the surrogate took this cycle
-  const int jj = bx * kPtBX + threadIdx.x;
-  const int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int nj = d.nj, ni = d.ni;
   if (jj >= nj || ii >= ni) return;
   const int k0 = bz * kKC, k1 = min(d.kz, k0 + kKC);
@@ -1460,7 +1490,7 @@ __device__ __forceinline__ void b_sound_momentum_km(const View<T>& d, const int 
 #define MOLOCH_KM_KERNELS(NAME)                                                                      \
   template <class T>                                                                                 \
   __global__ void __launch_bounds__(kPtBX* kPtBY) k_##NAME##_km(View<T> d) {                          \
-    b_##NAME##_km<T>(d, blockIdx.x, blockIdx.y, blockIdx.z);                                         \
+    b_##NAME##_km<T>(d, blockIdx.x, tile_y(d), blockIdx.z);                                         \
   }                                                                                                  \
   template <class T>                                                                                 \
   __global__ void __launch_bounds__(kPtBX* kPtBY)                                                    \
@@ -2790,8 +2820,8 @@ __device__ __forceinline__ void b_waf_vertical(const View<T>& d, const int bx, c
   constexpr int NG = kNumAdvected / F;
   const int g = bx % NG;
   const int tj = bx / NG;
-  const int jj = tj * kColBX + threadIdx.x;
-  const int ii = by * kColBY + threadIdx.y;
+  int jj, ii;
+  point_at<kColBX, kColBY>(d, tj, by, jj, ii);
   if (jj >= d.nj || ii >= d.ni) return;
   // the groups holding fields 2..4 (block-uniform branch)
   if constexpr (F == 1) {
@@ -3065,7 +3095,7 @@ constexpr int vert_min_blocks() {
 
 template <class T, int F>
 __global__ void __launch_bounds__(kColBX* kColBY, vert_min_blocks<T, F>()) k_waf_vertical(View<T> d) {
-  b_waf_vertical<T, F>(d, blockIdx.x, blockIdx.y, blockIdx.z);
+  b_waf_vertical<T, F>(d, blockIdx.x, tile_y(d), blockIdx.z);
 }
 
 template <class T, int F>
@@ -3577,8 +3607,9 @@ __device__ __forceinline__ f32x2 hflux2(const HFace2& f, float n0, float n1, f32
   return fma2(fma2(bb, f.zm, f.nis), d, add2(m1, x0));
 }
 constexpr int kHPairJ = 60;
+constexpr int kHPThreads = 128;  // 32 and 64 the same
 constexpr int kHPG = 5, kHPAhead = 1, kHPArrays = 2 * kHPG + 9;  // fields per warp, rows ahead
-constexpr int kHPSmem = (kHPAhead + 1) * kHPArrays * 128 * 8;
+constexpr int kHPSmem = (kHPAhead + 1) * kHPArrays * kHPThreads * 8;
 // a b, a product that no sum may absorb (the assembler fuses mul.rn.f32x2
 // with an add.rn.f32x2 that follows it)
 __device__ __forceinline__ f32x2 product2(f32x2 a, f32x2 b) {
@@ -3650,24 +3681,24 @@ __device__ __forceinline__ void b_waf_hpair(const View<float>& d, const int bx, 
     float2* const slot0 = hp_ring + threadIdx.x;
     auto fetch_row = [&](int i, int st) {
       if (i < i_e) {
-        float2* q = slot0 + st * (kHPArrays * 128);
+        float2* q = slot0 + st * (kHPArrays * kHPThreads);
         const unsigned r = row(i), rn = row(i + 1), r2 = row(i + 2);
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-          cp_async8(q + g * 128, wz[g] + r2);
-          cp_async8(q + (G + g) * 128, pp[g] + r);
+          cp_async8(q + g * kHPThreads, wz[g] + r2);
+          cp_async8(q + (G + g) * kHPThreads, pp[g] + r);
         }
-        q += 2 * G * 128;
+        q += 2 * G * kHPThreads;
         cp_async8(q, v + rn);
-        cp_async8(q + 128, wn_ + r);
-        cp_async8(q + 2 * 128, ws_ + r);
-        cp_async8(q + 3 * 128, u + r);
-        cp_async8(q + 4 * 128, we_ + r);
-        cp_async8(q + 5 * 128, ww_ + r);
-        cp_async8(q + 6 * 128, (ROT ? d.mu : d.rmu) + r);
+        cp_async8(q + kHPThreads, wn_ + r);
+        cp_async8(q + 2 * kHPThreads, ws_ + r);
+        cp_async8(q + 3 * kHPThreads, u + r);
+        cp_async8(q + 4 * kHPThreads, we_ + r);
+        cp_async8(q + 5 * kHPThreads, ww_ + r);
+        cp_async8(q + 6 * kHPThreads, (ROT ? d.mu : d.rmu) + r);
         if (!ROT) {
-          cp_async8(q + 7 * 128, d.rmv + rn);
-          cp_async8(q + 8 * 128, d.mx2 + r);
+          cp_async8(q + 7 * kHPThreads, d.rmv + rn);
+          cp_async8(q + 8 * kHPThreads, d.mx2 + r);
         }
       }
       cp_async_commit();
@@ -3679,11 +3710,11 @@ __device__ __forceinline__ void b_waf_hpair(const View<float>& d, const int bx, 
     for (int i = i_s; i < i_e; ++i) {
       const unsigned r = row(i);
       cp_async_wait<kHPAhead - 1>();
-      const float2* q = slot0 + rd * (kHPArrays * 128);
-      const float2* qs = q + 2 * G * 128;
-      const f32x2 vr = pack2(qs[0]), pn = pack2(qs[128]), ps = pack2(qs[2 * 128]), uu = pack2(qs[3 * 128]), oe = pack2(qs[4 * 128]),
-                  ow = pack2(qs[5 * 128]), zmf = pack2(qs[6 * 128]);
-      const f32x2 rmv = ROT ? neg : pack2(qs[7 * 128]), mx2 = ROT ? neg : pack2(qs[8 * 128]);
+      const float2* q = slot0 + rd * (kHPArrays * kHPThreads);
+      const float2* qs = q + 2 * G * kHPThreads;
+      const f32x2 vr = pack2(qs[0]), pn = pack2(qs[kHPThreads]), ps = pack2(qs[2 * kHPThreads]), uu = pack2(qs[3 * kHPThreads]), oe = pack2(qs[4 * kHPThreads]),
+                  ow = pack2(qs[5 * kHPThreads]), zmf = pack2(qs[6 * kHPThreads]);
+      const f32x2 rmv = ROT ? neg : pack2(qs[7 * kHPThreads]), mx2 = ROT ? neg : pack2(qs[8 * kHPThreads]);
       const f32x2 uz = mul2(uu, zmf);
       const f32x2 v_n = ROT ? vr : mul2(vr, rmv), uf = ROT ? uu : uz;
       const f32x2 mfac = ROT ? mul2(half, vr) : mul2(mul2(half, vr), rmv);
@@ -3697,7 +3728,7 @@ __device__ __forceinline__ void b_waf_hpair(const View<float>& d, const int bx, 
       const f32x2 odv = fma2(ufe, oe, mul2(uf, mul2(ow, neg)));
       f32x2 wp2[G], pold[G];
 #pragma unroll
-      for (int g = 0; g < G; ++g) { wp2[g] = pack2(q[g * 128]); pold[g] = pack2(q[(G + g) * 128]); }
+      for (int g = 0; g < G; ++g) { wp2[g] = pack2(q[g * kHPThreads]); pold[g] = pack2(q[(G + g) * kHPThreads]); }
       fetch_row(i + kHPAhead, rd == 0 ? kHPAhead : rd - 1);
 #pragma unroll
       for (int g = 0; g < G; ++g) {
@@ -3726,7 +3757,7 @@ __device__ __forceinline__ void b_waf_hpair(const View<float>& d, const int bx, 
   }
 }
 template <bool ROT>
-__global__ void __launch_bounds__(128, 3) k_waf_hpair(View<float> d) {
+__global__ void __launch_bounds__(kHPThreads, 384 / kHPThreads) k_waf_hpair(View<float> d) {
   constexpr int NG = kNumAdvected / kHPG;
   b_waf_hpair<ROT>(d, blockIdx.x / NG, blockIdx.y, (blockIdx.x % NG) * kHPG);
 }
@@ -3751,8 +3782,8 @@ __global__ void __launch_bounds__(128)
 // Writes u, v into buffer 0 so every step replays the same pointers.
 template <class T>
 __device__ __forceinline__ void b_stag_from_x(const View<T>& d, const int bx, const int by, const int bz) {
-  int jj = bx * kPtBX + threadIdx.x;
-  int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int nj = d.nj, ni = d.ni, kz = d.kz, kk = bz;
   if (jj >= nj || ii >= ni) return;
   // 32-bit element offsets: a field holds at most 2^31 points
@@ -3783,7 +3814,7 @@ __device__ __forceinline__ void b_stag_from_x(const View<T>& d, const int bx, co
 
 template <class T>
 __global__ void __launch_bounds__(kPtBX* kPtBY) k_stag_from_x(View<T> d) {
-  b_stag_from_x<T>(d, blockIdx.x, blockIdx.y, blockIdx.z);
+  b_stag_from_x<T>(d, blockIdx.x, tile_y(d), blockIdx.z);
 }
 
 // The same for FP32 storage with jx a multiple of 4 (View::stag4): each
@@ -3851,8 +3882,8 @@ __global__ void __launch_bounds__(kPtBX* kPtBY)
 // 46, 256 x 256 x 40 FP32 66 -> 31; 512 x 512 x 60 the same 0.145 ms.
 template <class T>
 __device__ __forceinline__ void b_postdiag(const View<T>& d, const int bx, const int by, const int bz) {
-  const int jj = bx * kPtBX + threadIdx.x;
-  const int ii = by * kPtBY + threadIdx.y;
+  int jj, ii;
+  point_at<kPtBX, kPtBY>(d, bx, by, jj, ii);
   const int nj = d.nj, ni = d.ni, kz = d.kz;
   if (jj >= nj || ii >= ni) return;
   const size_t pl = d.pl;
@@ -3880,7 +3911,7 @@ __device__ __forceinline__ void b_postdiag(const View<T>& d, const int bx, const
 
 template <class T>
 __global__ void __launch_bounds__(kPtBX* kPtBY) k_postdiag(View<T> d) {
-  b_postdiag<T>(d, blockIdx.x, blockIdx.y, blockIdx.z);
+  b_postdiag<T>(d, blockIdx.x, tile_y(d), blockIdx.z);
 }
 
 template <class T>
@@ -3988,13 +4019,15 @@ inline FieldPtrs<T> field_set(const View<T>& d, int set) {
 inline dim3 col_grid(int nj, int ni, int z = 1) {
   return dim3((nj + kColBX - 1) / kColBX, (ni + kColBY - 1) / kColBY, z);
 }
-inline dim3 pt_grid(int nj, int ni, int nz) {
-  return dim3((nj + kPtBX - 1) / kPtBX, (ni + kPtBY - 1) / kPtBY, nz);
+template <class T>
+dim3 pt_grid(const View<T>& d, int nz) {
+  if (in_order(d)) return dim3((unsigned)((d.pl + kPtBX * kPtBY - 1) / (kPtBX * kPtBY)), 1, nz);
+  return dim3((d.nj + kPtBX - 1) / kPtBX, (d.ni + kPtBY - 1) / kPtBY, nz);
 }
 
 template <class T>
 int launch_prediag(const View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
-  MOLOCH_LAUNCH(KK_PREDIAG, st, k_prediag<T><<<pt_grid(d.nj, d.ni, d.kz), dim3(kPtBX, kPtBY), 0, st>>>(d, fl.filterpai, fl.filtertheta));
+  MOLOCH_LAUNCH(KK_PREDIAG, st, k_prediag<T><<<pt_grid(d, d.kz), dim3(kPtBX, kPtBY), 0, st>>>(d, fl.filterpai, fl.filtertheta));
   return 1;
 }
 
@@ -4063,8 +4096,8 @@ inline int column_tw_grid(const View<T>& d) {
 template <class T>
 int launch_sound(View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
   int n = 0;
-  const dim3 pb(kPtBX, kPtBY), pg = pt_grid(d.nj, d.ni, d.kz);
-  const dim3 kg = pt_grid(d.nj, d.ni, (d.kz + kKC - 1) / kKC);  // k-marching: chunks of kKC levels
+  const dim3 pb(kPtBX, kPtBY), pg = pt_grid(d, d.kz);
+  const dim3 kg = pt_grid(d, (d.kz + kKC - 1) / kKC);  // k-marching: chunks of kKC levels
   for (int ns = 1; ns <= fl.nsound; ++ns) {
     const int last = ns == fl.nsound;
     // the fused strips recompute the divergence of a rim: bound by the FP64
@@ -4167,7 +4200,9 @@ int launch_sound(View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
 template <class T>
 void launch_waf_vertical(const View<T>& d, cudaStream_t st) {
   const int ng = kNumAdvected / d.vfields;
-  const dim3 vg(((d.nj + kColBX - 1) / kColBX) * ng, (d.ni + kColBY - 1) / kColBY), vb(kColBX, kColBY);
+  const dim3 vb(kColBX, kColBY);
+  const dim3 vg = in_order(d) ? dim3((unsigned)((d.pl + kColBX * kColBY - 1) / (kColBX * kColBY)) * ng)
+                              : dim3(((d.nj + kColBX - 1) / kColBX) * ng, (d.ni + kColBY - 1) / kColBY);
   // jx even: rows of column pairs (8-byte loads); faster at every size
   if constexpr (sizeof(T) == 4) {
     if (d.vfields == 1 && d.nj % 2 == 0) {
@@ -4201,7 +4236,7 @@ void blaunch_waf_vertical(const Batch<T>& b, const View<T>* views, cudaStream_t 
 // one advection() call; the advected fields move to the other buffer set
 template <class T>
 int launch_advection(View<T>& d, cudaStream_t st) {
-  const dim3 pb(kPtBX, kPtBY), pg = pt_grid(d.nj, d.ni, d.kz);
+  const dim3 pb(kPtBX, kPtBY), pg = pt_grid(d, d.kz);
   const dim3 hg((d.nj + 31) / 32, (d.ni + 7) / 8, (d.kz + d.hz_levels - 1) / d.hz_levels);
   launch_waf_vertical<T>(d, st);  // forms ux, vx, wx from u, v, w as well
   bool pairs = false;  // jx even: 8-byte loads of column pairs; faster at every size
@@ -4209,15 +4244,18 @@ int launch_advection(View<T>& d, cudaStream_t st) {
     pairs = d.hz_levels >= 16 && d.nj % 2 == 0;
     if (pairs) {
       const int np = ((d.nj + kHPairJ - 1) / kHPairJ) * ((d.ni + d.hz_levels - 1) / d.hz_levels);
-      const dim3 g((np + 3) / 4 * (kNumAdvected / kHPG), d.kz);
-      if (d.rotllr) MOLOCH_LAUNCH(KK_WAF_HORIZONTAL, st, k_waf_hpair<true><<<g, 128, kHPSmem, st>>>(d));
-      else MOLOCH_LAUNCH(KK_WAF_HORIZONTAL, st, k_waf_hpair<false><<<g, 128, kHPSmem, st>>>(d));
+      const dim3 g((np + kHPThreads / 32 - 1) / (kHPThreads / 32) * (kNumAdvected / kHPG), d.kz);
+      if (d.rotllr) MOLOCH_LAUNCH(KK_WAF_HORIZONTAL, st, k_waf_hpair<true><<<g, kHPThreads, kHPSmem, st>>>(d));
+      else MOLOCH_LAUNCH(KK_WAF_HORIZONTAL, st, k_waf_hpair<false><<<g, kHPThreads, kHPSmem, st>>>(d));
     }
   }
   if (pairs) {
   } else if (d.hz_levels >= 16) {  // warp strips of hz_levels rows
     const int nstrips = ((d.nj + kStripJ - 1) / kStripJ) * ((d.ni + d.hz_levels - 1) / d.hz_levels);
-    MOLOCH_LAUNCH(KK_WAF_HORIZONTAL, st, k_waf_hstrip<T><<<dim3((nstrips + 3) / 4, d.kz), 128, 0, st>>>(d));
+    // one warp a block, which balances a few hundred strips over the SMs: FP64
+    // at 100 x 100 x 30 0.547 (four) -> 0.430 ms per step; larger grids and FP32
+    // the same
+    MOLOCH_LAUNCH(KK_WAF_HORIZONTAL, st, k_waf_hstrip<T><<<dim3(nstrips, d.kz), 32, 0, st>>>(d));
   } else {
     MOLOCH_LAUNCH(KK_WAF_HORIZONTAL, st, k_waf_horizontal<T><<<hg, dim3(32, 8), 0, st>>>(d));
   }
@@ -4239,7 +4277,7 @@ int launch_advection(View<T>& d, cudaStream_t st) {
 template <class T>
 int launch_postdiag(View<T>& d, cudaStream_t st, const PhaseFlags& fl, const T* zk, const T* zkm1) {
   int n = 0;
-  const dim3 pb(kPtBX, kPtBY), pg = pt_grid(d.nj, d.ni, d.kz);
+  const dim3 pb(kPtBX, kPtBY), pg = pt_grid(d, d.kz);
   const size_t bytes = sizeof(T) * (size_t)d.pl * d.kz;
   if (fl.filterpai) {
     MOLOCH_LAUNCH(KK_FILTER_INCREMENT, st, k_filter_increment<T><<<pg, pb, 0, st>>>(d, 0));
