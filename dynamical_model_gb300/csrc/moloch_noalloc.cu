@@ -62,89 +62,18 @@ struct NaArgs {
 // 550 us, 64 x 48 x 30 226 -> 86 us, 200 x 190 x 20 574 -> 349 us, bit for bit
 // the same results.
 
-// 1 / b to half an ulp times 1 + 2^-11.6 (the estimate's third-order step,
-// rounded), and whether na_quot may use it.
-struct NaRcp {
-  double b, y;
-  bool ok;
-};
-__device__ __forceinline__ NaRcp na_rcp(double b) {
-  NaRcp r;
-  r.b = b;
-  r.ok = mid_range(b) && (__double2hiint(b) & 0xffe00) != 0xffe00;
-  const double x = rcp_seed(b), e = __fma_rn(-b, x, 1.0);
-  r.y = __fma_rn(x, __fma_rn(e, e, e), x);
-  return r;
-}
-// a / b, correctly rounded, with Markstein's quotient correction (P.
-// Markstein, "IA-64 and Elementary Functions", 2000): q = a y is within 1.5
-// ulp, the first residual takes it to half an ulp (1 + 2^-49), and the second
-// is exact, so that what is rounded last differs from a / b by at most
-// 2^-107 b (1 + 2^-11.5) where a >= b (a and b scaled to [1, 2)).  A quotient
-// of two doubles is no nearer than 2^-105 / b to the middle of two doubles:
-// the rounding is right while b < 2 (1 - 2^-12.5).  a < b halves both.  Other
-// b, and |a| outside 2^-800 .. 2^800 but 0, divide as IEEE.
-__device__ __forceinline__ double na_quot(double a, const NaRcp& r) {
-  const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
-  const bool zero = (h | (unsigned)__double2loint(a)) == 0u;
-  if (!(r.ok && (zero || h - 0x0df00000u < 0x71f00000u - 0x0df00000u))) return a / r.b;
-  double q = a * r.y;
-  q = __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
-  return __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
-}
-// 1 / b, correctly rounded (the same with q = y)
-__device__ __forceinline__ double na_inv(double b) {
-  const NaRcp r = na_rcp(b);
-  return r.ok ? __fma_rn(__fma_rn(-b, r.y, 1.0), r.y, r.y) : 1.0 / b;
-}
-// x / 2 by the exponent
-__device__ __forceinline__ double na_half(double x) {
-  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-  if (e - 2u < 0x7ffu - 2u) return __hiloint2double(__double2hiint(x) - 0x100000, __double2loint(x));
-  return 0.5 * x;
-}
-
-// superbee by the bits of r: 0 below 0, 2r up to 1/2, 1 up to 1, r up to 2,
-// then 2; 1 for NaN, as the comparisons of superbee() fall
-__device__ __forceinline__ double na_superbee(double r) {
-  const long long x = __double_as_longlong(r);
-  const long long half = 0x3fe0000000000000LL, one = 0x3ff0000000000000LL, two = 0x4000000000000000LL;
-  long long b = x < one ? one : x;
-  if (x < half) b = x >= 0x0010000000000000LL ? x + 0x0010000000000000LL : x << 1;  // subnormal: twice by a shift
-  if (x >= two) b = two;
-  if (x < 0) b = 0;
-  if ((x & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL) b = one;
-  return __longlong_as_double(b);
-}
-// sign(max(abs(z), minden), z) by the bits of z (NaN becomes minden)
-__device__ __forceinline__ double na_safeden(double z) {
-  const unsigned long long lo = (unsigned long long)__double_as_longlong(kMinden), inf = 0x7ff0000000000000ULL;
-  const unsigned long long x = (unsigned long long)__double_as_longlong(z);
-  unsigned long long m = x & 0x7fffffffffffffffULL;
-  if (m - lo > inf - lo) m = lo;
-  return __longlong_as_double((long long)(m | (x & 0x8000000000000000ULL)));
-}
-
-// (1 + zphi) m1 + (1 - zphi) x0 of the flux between cells m1 and x0; up: the
-// wind comes from m1's side, num the difference that side of it
-__device__ __forceinline__ double na_flux(bool up, double zamu, double num, double den, double m1, double x0) {
-  const double is = up ? 1.0 : -1.0;
-  const double b = na_superbee(na_quot(num, na_rcp(na_safeden(den))));
-  const double zphi = (is + zamu * b) - (up ? b : -b);
-  return (1.0 + zphi) * m1 + (1.0 - zphi) * x0;
-}
 // horizontal flux (:1088-1104); dm, d0, dp: the differences x(i) - x(i-1) at
 // the face before, this one and the next
 __device__ __forceinline__ double na_hflux(double zamu, double dm, double d0, double dp, double m1, double x0) {
   const bool up = __double_as_longlong(zamu) > 0;
-  return na_flux(up, zamu, up ? dm : dp, d0, m1, x0);
+  return waf_flux_rn(up, zamu, up ? dm : dp, d0, m1, x0);
 }
 // flux through the lower face of x1 (:966-1012); d0, d1, d2: x(k) - x(k+1)
 // above x1, below it and below x2
 __device__ __forceinline__ double na_vflux(double s1, double zamu, double d0, double d1, double d2, double x1, double x2) {
   const long long z = __double_as_longlong(zamu);
   const bool up = z >= 0 || z == (long long)0x8000000000000000ULL;
-  return na_half(s1) * na_flux(up, zamu, up ? d2 : d0, d1, x2, x1);
+  return half_of(s1) * waf_flux_rn(up, zamu, up ? d2 : d0, d1, x2, x1);
 }
 
 // Both vertical passes (:966-1072).  A warp holds 32 columns and up to
@@ -168,8 +97,8 @@ __global__ void __launch_bounds__(32 * kNaWarps) k_na_vertical(NaArgs a) {
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
     if (k0 < k1) {
-      NaRcp r0;
-      if (pass == 0) r0 = na_rcp(a.fmzf[c + k0 * pl]);
+      RcpRn r0;
+      if (pass == 0) r0 = rcp_rn_of(a.fmzf[c + k0 * pl]);
       double x1 = X(k0), x2 = X(k0 + 1), d0 = X(k0 - 1) - x1, d1 = x1 - x2;
       double s0 = a.s[c + k0 * pl], w0 = 0.0;
       if (k0 > 0) w0 = na_vflux(s0, s0 * a.dtrdz, X(k0 - 2) - X(k0 - 1), d0, d1, X(k0 - 1), x1);
@@ -181,9 +110,9 @@ __global__ void __launch_bounds__(32 * kNaWarps) k_na_vertical(NaArgs a) {
           const double w1 = k < kz - 1 ? na_vflux(s1, s1 * a.dtrdz, d0, d1, d2, x1, x2) : 0.0;
           if (pass == 0) {
             const double f = a.dtrdz * a.fmz[c + k * pl];
-            const NaRcp r1 = na_rcp(a.fmzf[c + (k + 1) * pl]);
-            zu[n] = na_quot(f, r0);
-            zd[n] = na_quot(f, r1);
+            const RcpRn r1 = rcp_rn_of(a.fmzf[c + (k + 1) * pl]);
+            zu[n] = quot_rn(f, r0);
+            zd[n] = quot_rn(f, r1);
             dv[n] = s0 * zu[n] - s1 * zd[n];
             r0 = r1;
           }
@@ -209,14 +138,14 @@ __device__ void na_vpass(const double* src, double* dst, const NaArgs& a, size_t
   const int kz = a.kz;
   double x1 = src[c], x2 = src[c + pl], d0 = 0.0, d1 = x1 - x2;
   double w0 = 0.0, s0 = a.s[c];
-  NaRcp r0 = na_rcp(a.fmzf[c]);
+  RcpRn r0 = rcp_rn_of(a.fmzf[c]);
   for (int k = 0; k < kz; ++k) {
     const size_t o = c + k * pl;
     const double s1 = a.s[o + pl], x3 = src[c + min(k + 2, kz - 1) * pl], d2 = x2 - x3;
     const double w1 = k < kz - 1 ? na_vflux(s1, s1 * a.dtrdz, d0, d1, d2, x1, x2) : 0.0;
     const double f = a.dtrdz * a.fmz[o];
-    const NaRcp r1 = na_rcp(a.fmzf[o + pl]);
-    const double zu = na_quot(f, r0), zd = na_quot(f, r1);
+    const RcpRn r1 = rcp_rn_of(a.fmzf[o + pl]);
+    const double zu = quot_rn(f, r0), zd = quot_rn(f, r1);
     dst[o] = ((x1 - w0 * zu) + w1 * zd) + (s0 * zu - s1 * zd) * x1;
     x1 = x2; x2 = x3; d0 = d1; d1 = d2; w0 = w1; s0 = s1; r0 = r1;
   }
@@ -245,31 +174,31 @@ __global__ void __launch_bounds__(128) k_na_meridional(NaArgs a) {
   auto face = [&](double v, double rm, double dm, double d0, double dp, double m1, double x0) {  // zpby
     const double vr = a.rotllr ? v : v * rm;
     const double fl = na_hflux(vr * a.dtrdy, dm, d0, dp, m1, x0);
-    return a.rotllr ? na_half(v) * fl : (na_half(v) * rm) * fl;
+    return a.rotllr ? half_of(v) * fl : (half_of(v) * rm) * fl;
   };
-  double rms = na_inv(a.mv[row(i0) + jj]);
+  double rms = inv_rn(a.mv[row(i0) + jj]);
   const double m2 = a.wz[ko + row(i0 - 2)], m1 = a.wz[ko + row(i0 - 1)];
   double x1 = a.wz[ko + row(i0)], x2 = a.wz[ko + row(i0 + 1)], d0 = x1 - m1, d1 = x2 - x1;
   double vs = a.v[ko + row(i0)], fc = a.fmz[ko + row(i0)];
   double zs = face(vs, rms, m1 - m2, d0, d1, m1, x1);
-  NaRcp rs = na_rcp(fc + a.fmz[ko + row(i0 - 1)]);
+  RcpRn rs = rcp_rn_of(fc + a.fmz[ko + row(i0 - 1)]);
   const double dt2 = a.dtrdy * 2.0;  // (c m) 2 f rounds as ((2 c) m) f
 #pragma unroll 1
   for (int i = i0; i < i1; ++i) {
     const size_t rc = row(i), rn = row(i + 1), rnn = row(i + 2);
-    const double rmn = na_inv(a.mv[rn + jj]), mxx = a.mx[rc + jj];
+    const double rmn = inv_rn(a.mv[rn + jj]), mxx = a.mx[rc + jj];
     const double hn = a.rotllr ? (dt2 * rmn) * mxx : mxx * mxx, hs = a.rotllr ? (dt2 * rms) * mxx : 0.0;
     const double x3 = a.wz[ko + rnn], vn = a.v[ko + rn], fn = a.fmz[ko + rn], pp = a.pp[ko + rc];
     const double d2 = x3 - x2, zn = face(vn, rmn, d0, d1, d2, x1, x2);
-    const NaRcp r = na_rcp(fc + fn);
+    const RcpRn r = rcp_rn_of(fc + fn);
     double p0;
     if (a.rotllr) {
-      const double zrfmn = na_quot(hn * fc, r), zrfms = na_quot(hs * fc, rs);
+      const double zrfmn = quot_rn(hn * fc, r), zrfms = quot_rn(hs * fc, rs);
       const double zdv = (vn * zrfmn - vs * zrfms) * pp;
       p0 = ((x1 + zs * zrfms) - zn * zrfmn) + zdv;
     } else {
       const double h = dt2 * fc;
-      const double zrfmn = na_quot(h, r), zrfms = na_quot(h, rs);
+      const double zrfmn = quot_rn(h, r), zrfms = quot_rn(h, rs);
       const double zdv = ((vn * rmn) * zrfmn - (vs * rms) * zrfms) * pp;
       p0 = x1 + hn * (((zs * zrfms) - zn * zrfmn) + zdv);
     }
@@ -298,7 +227,7 @@ __global__ void __launch_bounds__(kNaSeg) k_na_zonal(NaArgs a, int rows, int len
   const int jc = wrap2(jp, nj), jm = wm1(jc, nj), jm2 = wm1(jm, nj), je = wp1(jc, nj);
   double x1[kNaZonK], fc[kNaZonK], uw[kNaZonK];
   if (face) {
-    const double mu = a.mu[row + jc], m = a.rotllr ? mu : na_inv(mu);
+    const double mu = a.mu[row + jc], m = a.rotllr ? mu : inv_rn(mu);
     sm[t] = m;
 #pragma unroll
     for (int n = 0; n < kNaZonK; ++n) {
@@ -310,9 +239,9 @@ __global__ void __launch_bounds__(kNaSeg) k_na_zonal(NaArgs a, int rows, int len
       const double zamu = (u * m) * a.dtrdx;
       const bool up = __double_as_longlong(zamu) > 0;
       const double num = (up ? xw : a.p0[o + je]) - (up ? a.p0[o + jm2] : x1[n]);
-      const double fl = na_flux(up, zamu, num, x1[n] - xw, xw, x1[n]);
-      sz[n][t] = a.rotllr ? na_half(u) * fl : (na_half(u) * m) * fl;
-      const NaRcp y = na_rcp(fc[n] + a.fmz[o + jm]);
+      const double fl = waf_flux_rn(up, zamu, num, x1[n] - xw, xw, x1[n]);
+      sz[n][t] = a.rotllr ? half_of(u) * fl : (half_of(u) * m) * fl;
+      const RcpRn y = rcp_rn_of(fc[n] + a.fmz[o + jm]);
       sb[n][t] = y.b;
       sy[n][t] = y.y;
       sk[n][t] = y.ok;
@@ -327,16 +256,16 @@ __global__ void __launch_bounds__(kNaSeg) k_na_zonal(NaArgs a, int rows, int len
     if (n >= nk) break;
     const size_t o = (size_t)(kk + n) * pl + row;
     const double ue = a.u[o + je], pp = a.pp[o + jc];
-    const NaRcp re = {sb[n][e], sy[n][e], sk[n][e]}, rw = {sb[n][t], sy[n][t], sk[n][t]};
+    const RcpRn re = {sb[n][e], sy[n][e], sk[n][e]}, rw = {sb[n][t], sy[n][t], sk[n][t]};
     double out;
     if (a.rotllr) {
       const double h = (dt2 * m) * fc[n];
-      const double zrfme = na_quot(h, re), zrfmw = na_quot(h, rw);
+      const double zrfme = quot_rn(h, re), zrfmw = quot_rn(h, rw);
       const double zdv = (ue * zrfme - uw[n] * zrfmw) * pp;
       out = ((x1[n] + sz[n][t] * zrfmw) - sz[n][e] * zrfme) + zdv;
     } else {
       const double h = dt2 * fc[n];
-      const double zrfme = na_quot(h, re), zrfmw = na_quot(h, rw);
+      const double zrfme = quot_rn(h, re), zrfmw = quot_rn(h, rw);
       const double zdv = ((ue * me) * zrfme - (uw[n] * m) * zrfmw) * pp;
       out = x1[n] + (mx * mx) * (((sz[n][t] * zrfmw) - sz[n][e] * zrfme) + zdv);
     }
