@@ -65,28 +65,33 @@ ALG_WORDS = {
 # from an ncu capture of the kernel, and the grid points of that capture;
 # scaled by the point count to the benchmarked size (traffic grows in
 # proportion: one pass over each array per launch)
-NCU_TRAFFIC = {"k_sound_column": (847.0e6, 384 * 384 * 60), "k_sound_column_tm": (498.7e6, 384 * 384 * 60),
-               "k_sound_column_tw12": (531.8e6, 384 * 384 * 60)}
+_STAGED = (1055.7e6, 512 * 512 * 60)
+NCU_TRAFFIC = {"k_sound_column": (847.0e6, 384 * 384 * 60), "k_sound_column_tm": _STAGED,
+               "k_sound_column_tw12": _STAGED}
 # sm__pipe_fp64_cycles_active (% of peak, active) from the same captures
 NCU_FP64_PIPE = {"k_sound_column": {"pipe_fp64_active_pct": 35.7, "capture": "384x384x60",
                                     "fp64_operations_per_level": 4},
-                 "k_sound_column_tm": {"pipe_fp64_active_pct": 39.0, "capture": "384x384x60",
+                 "k_sound_column_tm": {"pipe_fp64_active_pct": 53.9, "capture": "512x512x60",
                                        "fp64_operations_per_level": 4},
-                 "k_sound_column_tw12": {"pipe_fp64_active_pct": 49.9, "capture": "384x384x60",
+                 "k_sound_column_tw12": {"pipe_fp64_active_pct": 53.9, "capture": "512x512x60",
                                          "fp64_operations_per_level": 4}}
 
 
 def column_variant(name, tuning):
-    """The staged column solve the tuning runs under the profile's kernel
-    kind k_sound_column_tm: bit 128 (with 32) the two-word kernel with 12
-    compute warps, bit 256 with 16, else the four-word kernel."""
+    """Name of the staged column solve under the profile's kernel kind
+    k_sound_column_tm, by the tuning's bits; all of them run the same kernel
+    (two words of column state a level, two CTAs an SM)."""
     if name != "k_sound_column_tm" or len(tuning) < 2:
         return name
     return "k_sound_column_tw12" if tuning[1] & 128 else "k_sound_column_tw16" if tuning[1] & 256 else name
-# the FP64 step's dominant kernels are bound by GB300's FP64 rate, not HBM:
-# their FP64-pipe activity from one-launch ncu captures at 256x256x60
-NCU_FP64_STEP = {"k_waf_vertical": {"pipe_fp64_active_pct": 84.3, "dram_pct": 2.0},
-                 "k_waf_horizontal": {"pipe_fp64_active_pct": 81.4, "dram_pct": 2.4}}
+# the FP64 step's kernels are bound by GB300's FP64 rate, not HBM: their
+# FP64-pipe activity from one-launch ncu captures at 256x256x60
+NCU_FP64_STEP = {"k_sound_column": {"pipe_fp64_active_pct": 83.3, "dram_pct": 20.3},
+                 "k_waf_vertical": {"pipe_fp64_active_pct": 71.7, "dram_pct": 7.1},
+                 "k_waf_horizontal": {"pipe_fp64_active_pct": 75.4, "dram_pct": 8.8},
+                 "k_sound_momentum": {"pipe_fp64_active_pct": 77.5, "dram_pct": 10.6},
+                 "k_sound_div": {"pipe_fp64_active_pct": 86.4, "dram_pct": 21.0},
+                 "k_sound_damp": {"pipe_fp64_active_pct": 85.9, "dram_pct": 26.8}}
 # whole-step algorithmic words per grid point of the fused design target
 # (pre-diag 11 + 3 sound cycles x 91 + 3 advection steps x 23 + post-diag 11)
 B_ALG_WORDS = 364
@@ -668,8 +673,8 @@ def run_single(args, dist, rank, ws, torch, dm, stream, local, device):
                 "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                 "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_ms,
                 "traffic": (NCU_TRAFFIC[tname][0] * gp / NCU_TRAFFIC[tname][1]) if tname in NCU_TRAFFIC else None,
-                "traffic_note": "ncu dram bytes of one launch at 384x384x60, scaled by grid points (part of the "
-                                "staged kernel's writes is still in L2 when it ends)",
+                "traffic_note": "ncu dram bytes of one launch (512x512x60; the one-thread solve 384x384x60), scaled "
+                                "by grid points (part of the writes is still in L2 when it ends)",
                 # second roof of the top kernel: its FP64 pivot recurrence (4
                 # FP64 operations per level) keeps the FP64 pipe this busy in
                 # the ncu capture of the same kernel

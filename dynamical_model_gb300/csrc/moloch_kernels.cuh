@@ -8,14 +8,18 @@
 //   k_prediag          :289-323  p, qsat, tvirt, qwltot, qwitot, tetav
 //   k_sound_div        :514-597  u/v halo + surface w + s (Eq. 10) + zdiv2 (Eq. 16)
 //   k_sound_damp       :853-895 + :627-630  divdamp and the vertical s term
-//   k_sound_column     :634-728  implicit w (Thomas, one thread per column),
+//   k_sound_column     :634-728  implicit w (Thomas; one thread per column, a block
+//                      per 8 to 32 columns (_split, FP64), or staged by TMA (_tw, FP32)),
 //                      Exner/theta update, nompi pai halo order, s completion (:843-849)
+//   k_divdamp_quad, _strip  div and damp in one pass (FP32)
 //   k_lap_filter       :423-440 divergence_filter (mo_divfilter)
 //   k_pai_update       :716-728 (split form used when the filter is on)
 //   k_sound_momentum   :730-837  Equations 17, 18
-//   k_waf_vertical     :966-1073  both vertical WAF passes in registers, all 10 fields,
+//   k_waf_vertical     :966-1073  both vertical WAF passes in registers, all 10 fields
+//                      (_pair: two columns per thread, FP32),
 //                      with (u,v,w) -> (ux,vx,wx) of :1327-1341, :1389-1417 formed on the fly
 //   k_waf_horizontal   :1075-1187 meridional + zonal WAF of one level, p0 in shared memory
+//                      (_hstrip: warp strips; _hpair: strips of two columns a lane, FP32)
 //   k_stag_from_x      :1343-1387  (ux,vx,wx) -> (u,v,w)
 //   k_filter_increment :442-481 + :333-353 filtpai / filttheta
 //   k_postdiag         :355-391  tvirt, t, p, rho, ps, qsat

@@ -117,13 +117,14 @@ struct View {
   T anu2;
 
   // launch shape chosen by the autotuner: levels per k_waf_horizontal block
-  int hz_levels;
+  int hz_levels;   // (16 and more: rows per warp strip)
   int kmarch;      // sound kernel variants, bit mask: 1 divergence, 2 damping, 4 momentum
                    // k-marching; 8 momentum as warp strips; 16 divergence + damping fused;
                    // 32 column solve staged by TMA with its column state in TMEM (128, 256
                    // with it: the same kernel); 64 with 8: momentum with four columns per
                    // thread (jx a multiple of 4) or strips with two columns per lane (jx
-                   // even); 512 with 16: the fused strips over two levels per warp
+                   // even); 512 with 16: four columns per thread (jx a multiple of 4) or
+                   // the fused strips over two levels per warp
   int vfields;     // advected fields per thread of k_waf_vertical: 1, 2, 5 or 10
   int srows;       // rows per warp strip of the momentum strips
   int stag4;       // 1: k_stag_from_x4 (FP32, jx a multiple of 4)

@@ -245,13 +245,14 @@ const char* moloch_gpu_kernel_name(int kind);
  * timed with CUDA events on the handle's stream and the fastest is kept
  * (moloch_gpu_tuning_count() slots):
  *   choice[0] = horizontal WAF kernel: 1, 2, 4, 8 levels per 32x8 tile
- *               block, or 16, 32, 64 rows per warp strip;
+ *               block, or 16, 32, 64 rows per warp strip (FP32 storage with
+ *               even jx: two columns per lane, not in ensembles);
  *   choice[1] = sound kernel variants, bit mask: 1 divergence, 2 damping,
  *               4 momentum as k-marching kernels (chunks of 4 levels per
  *               thread, next level prefetched), 8 momentum as warp strips
  *               (30 columns x 32 rows), 16 divergence and damping fused in
  *               one warp-strip kernel (29 columns x 32 rows; overrides 1
- *               and 2; MOLOCH_FP64 ignores it), 32 the implicit-w column
+ *               and 2; MOLOCH_FP64 runs its separate kernels), 32 the implicit-w column
  *               solve staged by TMA with its column state in TMEM (FP32
  *               storage, jx a multiple of 4, kz <= 64; elsewhere the bit is
  *               ignored), 64 (with 8) the momentum with four columns per
@@ -260,13 +261,14 @@ const char* moloch_gpu_kernel_name(int kind);
  *               ensembles, the one-column strips; 128 or 256 (with 32, not
  *               both, and not in ensembles): once other shapes of the
  *               staged column solve, now the same kernel; 512 (with 16) the
- *               fused
- *               divergence/damping strips over two levels per warp
- *               (shared row loads; not in ensembles); 0 = one level per
- *               thread;
+ *               divergence and damping with four columns per thread (FP32
+ *               storage, jx a multiple of 4, kz <= 512), elsewhere the fused
+ *               strips over two levels per warp (not in ensembles); 0 = one
+ *               level per thread;
  *   choice[2] = advected fields per thread of the vertical WAF kernel:
  *               1, 2, 5 or 10 (the fields of a thread share the velocity
- *               loads and terms);
+ *               loads and terms; 1 in FP32 storage with even jx: two columns
+ *               per thread, not in ensembles);
  *   choice[3] = rows per warp strip of the momentum strips, 4 to 64
  *               (candidates 4, 8, 16, 32: shorter strips put more warps in
  *               flight; in ensembles the one-launch-per-kernel mode takes
