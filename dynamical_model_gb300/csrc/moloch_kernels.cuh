@@ -263,6 +263,7 @@ __device__ __forceinline__ double pow35(double a) {
 __device__ __forceinline__ double qdiv(double a, double b) { return div_nr(a, b); }
 __device__ __forceinline__ double pow_cpovr(double a) { return pow35(a); }
 #else
+__device__ __forceinline__ double qdiv(double a, double b) { return a / b; }
 __device__ __forceinline__ double pow_cpovr(double a) { return pow(a, kCpovr); }
 #endif
 __device__ __forceinline__ float pow_cpovr(float a) { return powf(a, (float)kCpovr); }
