@@ -2575,14 +2575,16 @@ __device__ __forceinline__ RcpRn rcp_rn_of(double b) {
 // 2^-107 b (1 + 2^-11.5) where a >= b (a and b scaled to [1, 2)).  A quotient
 // of two doubles is no nearer than 2^-105 / b to the middle of two doubles:
 // the rounding is right while b < 2 (1 - 2^-12.5).  a < b halves both.  Other
-// b, and |a| outside 2^-800 .. 2^800 but 0, divide as IEEE.
+// b, and |a| outside 2^-800 .. 2^800 but 0, divide as IEEE.  A zero's first
+// product has the quotient's sign; the residuals would turn -0 into +0.
 __device__ __forceinline__ double quot_rn(double a, const RcpRn& r) {
   const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
   const bool zero = (h | (unsigned)__double2loint(a)) == 0u;
   if (!(r.ok && (zero || h - 0x0df00000u < 0x71f00000u - 0x0df00000u))) return a / r.b;
-  double q = a * r.y;
+  const double q0 = mul_rn(a, r.y);
+  double q = __fma_rn(__fma_rn(-r.b, q0, a), r.y, q0);
   q = __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
-  return __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
+  return zero ? q0 : q;
 }
 // 1 / b, correctly rounded (the same with q = y)
 __device__ __forceinline__ double inv_rn(double b) {

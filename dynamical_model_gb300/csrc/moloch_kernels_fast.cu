@@ -118,6 +118,16 @@ __global__ void k_check_division_f64(const double* __restrict__ a, const double*
     qi[q] = a[q] / b[q];
   }
 }
+__global__ void k_check_math_f64(int op, const double* __restrict__ a, const double* __restrict__ b,
+                                 double* __restrict__ out, double* __restrict__ ref, int n) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const double x = a[q], y = b[q];
+    switch (op) {
+      case 0: out[q] = quot_rn(x, rcp_rn_of(y)); ref[q] = x / y; break;
+      default: out[q] = inv_rn(y); ref[q] = 1.0 / y; break;
+    }
+  }
+}
 }  // namespace kfast
 }  // namespace moloch
 
@@ -137,5 +147,13 @@ extern "C" int moloch_gpu_check_division_f64(const double* a, const double* b, d
   if (n == 0) return MOLOCH_OK;
   const int blocks = (n + 255) / 256 < 1024 ? (n + 255) / 256 : 1024;
   moloch::kfast::k_check_division_f64<<<blocks, 256, 0, (cudaStream_t)stream>>>(a, b, q_nr, q_ieee, n);
+  return cudaPeekAtLastError() == cudaSuccess ? MOLOCH_OK : MOLOCH_ERR_CUDA;
+}
+extern "C" int moloch_gpu_check_math_f64(int op, const double* a, const double* b, double* out, double* ref, int n,
+                                         void* stream) {
+  if (op < 0 || op > 1 || !a || !b || !out || !ref || n < 0) return MOLOCH_ERR_ARG;
+  if (n == 0) return MOLOCH_OK;
+  const int blocks = (n + 255) / 256 < 1024 ? (n + 255) / 256 : 1024;
+  moloch::kfast::k_check_math_f64<<<blocks, 256, 0, (cudaStream_t)stream>>>(op, a, b, out, ref, n);
   return cudaPeekAtLastError() == cudaSuccess ? MOLOCH_OK : MOLOCH_ERR_CUDA;
 }

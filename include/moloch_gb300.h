@@ -219,6 +219,15 @@ int moloch_gpu_check_division(const float* a, const float* b, float* q_corr, flo
 int moloch_gpu_check_division_f64(const double* a, const double* b, double* q_nr, double* q_ieee, int n,
                                   void* stream);
 
+/* Arithmetic check (tests) of the other FP64 operations the kernels write
+ * out themselves, beside CUDA's own (ref), for n device values:
+ *   op 0  the quotient a / b from a shared reciprocal (exact build's WAF
+ *         values and one-field advection) against a / b;
+ *   op 1  the reciprocal 1 / b there.
+ * No reference counterpart. */
+int moloch_gpu_check_math_f64(int op, const double* a, const double* b, double* out, double* ref, int n,
+                              void* stream);
+
 /* The stream the handle launches on (a cudaStream_t). */
 void* moloch_gpu_stream(moloch_handle_t* h);
 
