@@ -209,7 +209,7 @@ __device__ __forceinline__ float narrow_trunc(double x) {
 }
 
 
-// ---- FP64 quotients and roots of the contracting builds ----------------
+// ---- FP64 quotients and roots written out --------------------------------
 // FP32 estimate of 1 / b for |b| in the FP32 normal range (relative error
 // below 2^-21.9: the estimate's ulp and b cut to 23 bits)
 __device__ __forceinline__ double rcp_seed(double b) {
@@ -223,17 +223,45 @@ __device__ __forceinline__ bool mid_range(double b) {
   const unsigned h = (unsigned)__double2hiint(b) & 0x7fffffffu;
   return h - 0x39b00000u < 0x46300000u - 0x39b00000u;
 }
-// a / b in five FP64 operations: q = a x with the estimate x of 1 / b, then
-// twice q + (a - b q) x (Markstein's quotient correction, P. Markstein, "IA-64
-// and Elementary Functions", 2000), each of which multiplies the relative
-// error by 2^-21.9: within one ulp of the IEEE quotient.  Other b divide as
-// IEEE.
-__device__ __forceinline__ double div_nr(double a, double b) {
-  if (!mid_range(b)) return a / b;
-  const double x = rcp_seed(b);
-  double q = mul_rn(a, x);
-  q = fma_rn(fma_rn(-b, q, a), x, q);
-  return fma_rn(fma_rn(-b, q, a), x, q);
+// 1 / b to half an ulp times 1 + 2^-11.6 (the estimate's third-order step,
+// rounded), and whether quot_rn may use it.
+struct RcpRn {
+  double b, y;
+  bool ok;
+};
+__device__ __forceinline__ RcpRn rcp_rn_of(double b) {
+  RcpRn r;
+  r.b = b;
+  r.ok = mid_range(b) && (__double2hiint(b) & 0xffe00) != 0xffe00;
+  const double x = rcp_seed(b), e = __fma_rn(-b, x, 1.0);
+  r.y = __fma_rn(x, __fma_rn(e, e, e), x);
+  return r;
+}
+// a / b, correctly rounded, with Markstein's quotient correction (P.
+// Markstein, "IA-64 and Elementary Functions", 2000): q = a y is within 1.5
+// ulp, the first residual takes it to half an ulp (1 + 2^-49), and the second
+// is exact, so that what is rounded last differs from a / b by at most
+// 2^-107 b (1 + 2^-11.5) where a >= b (a and b scaled to [1, 2)).  A quotient
+// of two doubles is no nearer than 2^-105 / b to the middle of two doubles:
+// the rounding is right while b < 2 (1 - 2^-12.5).  a < b halves both.  Other
+// b, and |a| outside 2^-800 .. 2^800 but 0, divide as IEEE.  A zero's first
+// product has the quotient's sign; the residuals would turn -0 into +0.
+// Eight FP64 operations with the reciprocal.  (Two corrections of a y from the
+// estimate itself are five, but only within an ulp, and make NaN of infinite
+// and overflowing quotients.)
+__device__ __forceinline__ double quot_rn(double a, const RcpRn& r) {
+  const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  const bool zero = (h | (unsigned)__double2loint(a)) == 0u;
+  if (!(r.ok && (zero || h - 0x0df00000u < 0x71f00000u - 0x0df00000u))) return a / r.b;
+  const double q0 = mul_rn(a, r.y);
+  double q = __fma_rn(__fma_rn(-r.b, q0, a), r.y, q0);
+  q = __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
+  return zero ? q0 : q;
+}
+// 1 / b, correctly rounded (the same with q = y)
+__device__ __forceinline__ double inv_rn(double b) {
+  const RcpRn r = rcp_rn_of(b);
+  return r.ok ? __fma_rn(__fma_rn(-b, r.y, 1.0), r.y, r.y) : 1.0 / b;
 }
 // 1 / b in three: x + x (e + e^2) with e = 1 - b x (the third-order step of
 // the geometric series of 1 / (1 - e); relative error 2^-65 before rounding)
@@ -245,7 +273,7 @@ __device__ __forceinline__ double rcp_nr(double b) {
 // pai^3.5 = pai^3 sqrt(pai), the root by the coupled iteration for g =
 // sqrt(a), h = 1 / (2 sqrt(a)) (Goldschmidt's, as in Markstein's book) from an
 // FP32 estimate and a last correction g + (a - g^2) h: nine FP64 operations
-// where pow takes about seventy (256 x 256 x 60, with div_nr: k_prediag 0.93 ->
+// where pow takes about seventy (256 x 256 x 60, with quot_rn: k_prediag 0.93 ->
 // 0.33 ms, k_postdiag 1.14 -> 0.42 ms)
 __device__ __forceinline__ double pow35(double a) {
   static_assert(kCpovr - 3.5 < 1e-15 && 3.5 - kCpovr < 1e-15, "cp / R");
@@ -260,7 +288,7 @@ __device__ __forceinline__ double pow35(double a) {
   return mul_rn(mul_rn(mul_rn(a, a), a), g);
 }
 #if defined(MOLOCH_LEAN_FP64)
-__device__ __forceinline__ double qdiv(double a, double b) { return div_nr(a, b); }
+__device__ __forceinline__ double qdiv(double a, double b) { return quot_rn(a, rcp_rn_of(b)); }
 __device__ __forceinline__ double pow_cpovr(double a) { return pow35(a); }
 #else
 __device__ __forceinline__ double qdiv(double a, double b) { return a / b; }
@@ -801,7 +829,7 @@ __device__ __forceinline__ void b_sound_column_lean(const View<double>& d, const
     x.zd = ZD[q]; x.fz = FZD[q]; x.tet = TET[q]; x.pai = PAI[q];
     if (first) {
       const double qv = QV[q], qc = QC[q];
-      x.m1 = div_nr(fma(3.2, qc, fma(0.86, qv, 1.0)), fma(4.8, qc, fma(0.96, qv, 1.0)));
+      x.m1 = qdiv(fma(3.2, qc, fma(0.86, qv, 1.0)), fma(4.8, qc, fma(0.96, qv, 1.0)));
       x.m2 = fma(2.1, QWI[q], fma(4.2, QWL[q], 0.25 * qv));
     } else {
       x.m1 = MO1[q]; x.m2 = MO2[q];
@@ -1004,7 +1032,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4)
       double m1, m2;
       if (nsound == 1) {
         const double qv = QV[q], qc = QC[q];
-        m1 = div_nr(fma(3.2, qc, fma(0.86, qv, 1.0)), fma(4.8, qc, fma(0.96, qv, 1.0)));
+        m1 = qdiv(fma(3.2, qc, fma(0.86, qv, 1.0)), fma(4.8, qc, fma(0.96, qv, 1.0)));
         m2 = fma(2.1, QWI[q], fma(4.2, QWL[q], 0.25 * qv));
         d.mo1[c + q] = m1;
         d.mo2[c + q] = m2;
@@ -2549,48 +2577,11 @@ inline void dq_attributes() {
 }
 
 // ---- FP64 WAF value with the reference's rounding in fewer FP64 operations ----
-// (the exact build and the one-field advection): quotients from an FP32
-// estimate that round as IEEE, sign, order, halving and doubling by the bits.
+// (the exact build and the one-field advection): quotients that round as IEEE
+// (quot_rn), sign, order, halving and doubling by the bits.
 // Bound by the FP64 pipe (16 clocks a warp instruction).  Exact build, 53 x 47 x
 // 21, ms per step: vertical 0.464 -> 0.346, horizontal 0.479 -> 0.356, the same
 // bits.
-// 1 / b to half an ulp times 1 + 2^-11.6 (the estimate's third-order step,
-// rounded), and whether quot_rn may use it.
-struct RcpRn {
-  double b, y;
-  bool ok;
-};
-__device__ __forceinline__ RcpRn rcp_rn_of(double b) {
-  RcpRn r;
-  r.b = b;
-  r.ok = mid_range(b) && (__double2hiint(b) & 0xffe00) != 0xffe00;
-  const double x = rcp_seed(b), e = __fma_rn(-b, x, 1.0);
-  r.y = __fma_rn(x, __fma_rn(e, e, e), x);
-  return r;
-}
-// a / b, correctly rounded, with Markstein's quotient correction (P.
-// Markstein, "IA-64 and Elementary Functions", 2000): q = a y is within 1.5
-// ulp, the first residual takes it to half an ulp (1 + 2^-49), and the second
-// is exact, so that what is rounded last differs from a / b by at most
-// 2^-107 b (1 + 2^-11.5) where a >= b (a and b scaled to [1, 2)).  A quotient
-// of two doubles is no nearer than 2^-105 / b to the middle of two doubles:
-// the rounding is right while b < 2 (1 - 2^-12.5).  a < b halves both.  Other
-// b, and |a| outside 2^-800 .. 2^800 but 0, divide as IEEE.  A zero's first
-// product has the quotient's sign; the residuals would turn -0 into +0.
-__device__ __forceinline__ double quot_rn(double a, const RcpRn& r) {
-  const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
-  const bool zero = (h | (unsigned)__double2loint(a)) == 0u;
-  if (!(r.ok && (zero || h - 0x0df00000u < 0x71f00000u - 0x0df00000u))) return a / r.b;
-  const double q0 = mul_rn(a, r.y);
-  double q = __fma_rn(__fma_rn(-r.b, q0, a), r.y, q0);
-  q = __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
-  return zero ? q0 : q;
-}
-// 1 / b, correctly rounded (the same with q = y)
-__device__ __forceinline__ double inv_rn(double b) {
-  const RcpRn r = rcp_rn_of(b);
-  return r.ok ? __fma_rn(__fma_rn(-b, r.y, 1.0), r.y, r.y) : 1.0 / b;
-}
 // x / 2 by the exponent
 __device__ __forceinline__ double half_of(double x) {
   const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;

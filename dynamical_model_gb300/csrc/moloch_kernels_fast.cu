@@ -114,7 +114,7 @@ __global__ void k_check_division(const float* __restrict__ a, const float* __res
 __global__ void k_check_division_f64(const double* __restrict__ a, const double* __restrict__ b,
                                      double* __restrict__ qn, double* __restrict__ qi, int n) {
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-    qn[q] = qdiv(a[q], b[q]);  // div_nr in this build
+    qn[q] = qdiv(a[q], b[q]);  // quot_rn in this build
     qi[q] = a[q] / b[q];
   }
 }

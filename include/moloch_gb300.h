@@ -212,10 +212,10 @@ int moloch_gpu_set_wait_limit(moloch_handle_t* h, long long cycles, int skip_job
  * counterpart. */
 int moloch_gpu_check_division(const float* a, const float* b, float* q_corr, float* q_ieee, int n, void* stream);
 
-/* The same for FP64 (tests): q_nr = the quotient the contracting build's
- * diagnostics and column solve use (FP32 reciprocal estimate, two residual
- * corrections) and q_ieee = CUDA's IEEE FP64 quotient.  No reference
- * counterpart. */
+/* The same for FP64 (tests): q_nr = the quotient of the contracting build's
+ * diagnostics and moist factors (FP32 reciprocal estimate, residual
+ * corrections; rounds as IEEE) and q_ieee = CUDA's IEEE FP64 quotient.  No
+ * reference counterpart. */
 int moloch_gpu_check_division_f64(const double* a, const double* b, double* q_nr, double* q_ieee, int n,
                                   void* stream);
 

@@ -1,11 +1,12 @@
 """The FP64 operations the kernels write out themselves, against CUDA's.
 
-Quotients and reciprocals -- the shared-reciprocal quotient of the exact
-build's WAF values and of the one-field advection -- round as IEEE: the same
-bits (any NaN for a NaN) on seeded values, on denominators with mantissas on
-both sides of the cut below 2 where the short form ends, numerators beside
-multiples of them, the ends of the exponent ranges, zeros of both signs,
-subnormals, infinities and NaN.
+Quotients and reciprocals -- the diagnostics' and the moist factors' (the
+contracting build), the shared-reciprocal quotient of the exact build's WAF
+values and of the one-field advection -- round as IEEE: the same bits (any NaN
+for a NaN) on seeded values, on denominators with mantissas on both sides of
+the cut below 2 where the short form ends, numerators beside multiples of
+them, the ends of the exponent ranges, zeros of both signs, subnormals,
+infinities and NaN.
 """
 import ctypes
 
@@ -18,13 +19,15 @@ QUOT, INV = range(2)
 
 
 def check(dm, op, a, b):
-    """(the kernels' values, CUDA's)"""
+    """(the kernels' values, CUDA's); op None: the diagnostics' quotient"""
     torch = pytest.importorskip("torch")
     L = dm.lib()
     ta, tb = (torch.from_numpy(np.ascontiguousarray(x, dtype=np.float64)).to("cuda") for x in (a, b))
     out, ref = torch.empty_like(ta), torch.empty_like(ta)
     P = [ctypes.c_void_p(t.data_ptr()) for t in (ta, tb, out, ref)]
-    assert L.moloch_gpu_check_math_f64(op, *P, ta.numel(), None) == 0
+    rc = (L.moloch_gpu_check_division_f64(*P, ta.numel(), None) if op is None else
+          L.moloch_gpu_check_math_f64(op, *P, ta.numel(), None))
+    assert rc == 0
     torch.cuda.synchronize()
     return out.cpu().numpy(), ref.cpu().numpy()
 
@@ -70,7 +73,7 @@ def report(x, y, a, b):
     return f"{bad.size} of {x.size}; first: {a[bad[:3]]} / {b[bad[:3]]} -> {x[bad[:3]]}, IEEE {y[bad[:3]]}"
 
 
-@pytest.mark.parametrize("op", [QUOT])
+@pytest.mark.parametrize("op", [None, QUOT])
 def test_quotients_round_as_ieee(gpu_lib, op):
     b = denominators()
     for a in numerators(b):
@@ -85,7 +88,7 @@ def test_quotients_round_as_ieee(gpu_lib, op):
         assert same_bits(x, y).all(), report(x, y, a, b)
 
 
-@pytest.mark.parametrize("op", [QUOT])
+@pytest.mark.parametrize("op", [None, QUOT])
 def test_quotients_of_zeros_infinities_and_nan(gpu_lib, op):
     a, b = (x.ravel() for x in np.meshgrid(SPECIAL, SPECIAL))
     x, y = check(gpu_lib, op, a, b)
@@ -99,3 +102,21 @@ def test_reciprocals_round_as_ieee(gpu_lib, op):
     for b in (denominators(), SPECIAL, 1.0 + 10.0 ** r.uniform(-3, 3, n), 2.0 ** r.uniform(-99, 99, n)):
         x, y = check(gpu_lib, op, b, b)
         assert same_bits(x, y).all(), report(x, y, np.ones_like(b), b)
+
+
+@pytest.mark.parametrize("plant", [np.inf, -np.inf])
+def test_an_infinite_temperature_gives_the_quotient_ieee_gives(gpu_lib, plant):
+    """tetav = tvirt / pai of the pre-diagnostics, exact and contracting build"""
+    out = {}
+    for mode in ("fp64_exact", "fp64"):
+        g = gpu_lib.Moloch(9, 8, 5, mode=mode)
+        g.setup_idealized(hills=((300.0, 4.0, 4.0, 3.0),))
+        t = g.download("t")
+        t[3, 4, 2] = plant
+        g.upload("t", t)
+        g.phase(0)
+        out[mode] = g.get("tetav")
+        g.close()
+    assert np.isinf(out["fp64_exact"]).sum() == 1
+    assert np.array_equal(np.isinf(out["fp64"]), np.isinf(out["fp64_exact"]))
+    assert not np.isnan(out["fp64"]).any()
