@@ -151,16 +151,25 @@ __device__ __forceinline__ int wp1(int x, int n) { return x == n - 1 ? 0 : x + 1
 __device__ __forceinline__ int wm2(int x, int n) { int y = x - 2; return y < 0 ? y + n : y; }
 __device__ __forceinline__ int wp2(int x, int n) { int y = x + 2; return y >= n ? y - n : y; }
 
-// a*b - c*d and a*b + c*d with the multiply-add contraction fixed in FP32
-// storage: left to the compiler either product may be fused, and which one
-// it fuses depends on the code around the expression, so the same body in
+// a*b - c*d and a*b + c*d with the multiply-add contraction fixed in the builds
+// that contract: left to the compiler either product may be fused, and which
+// one it fuses depends on the code around the expression, so the same body in
 // two kernels (k_sound_column and k_sound_column_tw; a batched kernel and
-// the persistent ensemble kernel) could round differently.  FP64 keeps the
-// expression as written (the exact build contracts nothing).
+// the persistent ensemble kernel) could round differently.  The exact build
+// contracts nothing.
 __device__ __forceinline__ float prod_sub(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
-__device__ __forceinline__ double prod_sub(double a, double b, double c, double d) { return a * b - c * d; }
 __device__ __forceinline__ float prod_add(float a, float b, float c, float d) { return __fmaf_rn(c, d, __fmul_rn(a, b)); }
+#if defined(MOLOCH_LEAN_FP64)
+__device__ __forceinline__ double prod_sub(double a, double b, double c, double d) { return __fma_rn(a, b, -__dmul_rn(c, d)); }
+__device__ __forceinline__ double prod_add(double a, double b, double c, double d) { return __fma_rn(c, d, __dmul_rn(a, b)); }
+#else
+__device__ __forceinline__ double prod_sub(double a, double b, double c, double d) { return a * b - c * d; }
 __device__ __forceinline__ double prod_add(double a, double b, double c, double d) { return a * b + c * d; }
+#endif
+// the fourth-order average of the staggering (:1327-1417) of the inner pair's
+// sum and the outer pair's, likewise fixed in FP64
+__device__ __forceinline__ float average4(float inner, float outer) { return 0.5625f * inner - 0.0625f * outer; }
+__device__ __forceinline__ double average4(double inner, double outer) { return prod_sub(0.5625, inner, 0.0625, outer); }
 __device__ __forceinline__ int wrapn(int x, int n) { int y = x % n; return y < 0 ? y + n : y; }
 // periodic index for -n <= x < 2n (no integer division)
 __device__ __forceinline__ int wrap2(int x, int n) { return x < 0 ? x + n : (x >= n ? x - n : x); }
@@ -2745,11 +2754,11 @@ __device__ __forceinline__ void b_waf_vertical_g(const View<T>& d, const int g, 
       T x;
       if (f == 2) {
         const T* __restrict__ us = d.ubuf[d.cur] + (o + (unsigned)nj * ii);
-        x = T(0.5625) * (us[wp1(jj, nj)] + us[jj]) - T(0.0625) * (us[wp2(jj, nj)] + us[wm1(jj, nj)]);
+        x = average4(us[wp1(jj, nj)] + us[jj], us[wp2(jj, nj)] + us[wm1(jj, nj)]);
       } else if (f == 3) {
         const T* __restrict__ vs = d.vbuf[d.cur] + (o + jj);
-        x = T(0.5625) * (vs[(unsigned)nj * wp1(ii, ni)] + vs[(unsigned)nj * ii]) -
-            T(0.0625) * (vs[(unsigned)nj * wp2(ii, ni)] + vs[(unsigned)nj * wm1(ii, ni)]);
+        x = average4(vs[(unsigned)nj * wp1(ii, ni)] + vs[(unsigned)nj * ii],
+                     vs[(unsigned)nj * wp2(ii, ni)] + vs[(unsigned)nj * wm1(ii, ni)]);
       } else if (f == 4) {
         const T* __restrict__ w = d.w + c;
         if (kk == 0)
@@ -2757,7 +2766,7 @@ __device__ __forceinline__ void b_waf_vertical_g(const View<T>& d, const int g, 
         else if (kk == kz - 1)
           x = T(0.5) * (w[(unsigned)kz * pl] + w[(unsigned)(kz - 1) * pl]);
         else
-          x = T(0.5625) * (w[(kk + 1) * pl] + w[kk * pl]) - T(0.0625) * (w[(kk + 2) * pl] + w[(kk - 1) * pl]);
+          x = average4(w[(kk + 1) * pl] + w[kk * pl], w[(kk + 2) * pl] + w[(kk - 1) * pl]);
       } else {
         return src[u][c + o];
       }
@@ -3843,10 +3852,10 @@ __device__ __forceinline__ void b_stag_from_x(const View<T>& d, const int bx, co
   const unsigned rowj = (unsigned)nj * (unsigned)ii;
   const T* __restrict__ ux = d.ux;
   const T* __restrict__ vx = d.vx;
-  d.ubuf[0][o + c] = T(0.5625) * (ux[o + c] + ux[o + rowj + wm1(jj, nj)]) -
-                     T(0.0625) * (ux[o + rowj + wp1(jj, nj)] + ux[o + rowj + wm2(jj, nj)]);
-  d.vbuf[0][o + c] = T(0.5625) * (vx[o + c] + vx[o + jj + (unsigned)nj * wm1(ii, ni)]) -
-                     T(0.0625) * (vx[o + jj + (unsigned)nj * wp1(ii, ni)] + vx[o + jj + (unsigned)nj * wm2(ii, ni)]);
+  d.ubuf[0][o + c] = average4(ux[o + c] + ux[o + rowj + wm1(jj, nj)],
+                              ux[o + rowj + wp1(jj, nj)] + ux[o + rowj + wm2(jj, nj)]);
+  d.vbuf[0][o + c] = average4(vx[o + c] + vx[o + jj + (unsigned)nj * wm1(ii, ni)],
+                              vx[o + jj + (unsigned)nj * wp1(ii, ni)] + vx[o + jj + (unsigned)nj * wm2(ii, ni)]);
   // w(k), k = 2..kz (1-based) <- wx ; level index kk = k-1 in 1..kz-1
   if (kk >= 1) {
     const T* __restrict__ wx = d.wx;
@@ -3856,8 +3865,7 @@ __device__ __forceinline__ void b_stag_from_x(const View<T>& d, const int bx, co
     else if (kk == kz - 1)
       wv = T(0.5) * (wx[c + (unsigned)(kz - 1) * pl] + wx[c + (unsigned)(kz - 2) * pl]);
     else
-      wv = T(0.5625) * (wx[c + kk * pl] + wx[c + (kk - 1) * pl]) -
-           T(0.0625) * (wx[c + (kk + 1) * pl] + wx[c + (kk - 2) * pl]);
+      wv = average4(wx[c + kk * pl] + wx[c + (kk - 1) * pl], wx[c + (kk + 1) * pl] + wx[c + (kk - 2) * pl]);
     d.w[c + kk * pl] = wv;
   }
 }
