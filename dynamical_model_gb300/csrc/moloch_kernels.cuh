@@ -272,13 +272,11 @@ __device__ __forceinline__ double inv_rn(double b) {
   const RcpRn r = rcp_rn_of(b);
   return r.ok ? __fma_rn(__fma_rn(-b, r.y, 1.0), r.y, r.y) : 1.0 / b;
 }
-// 1 / b in three: x + x (e + e^2) with e = 1 - b x (the third-order step of
-// the geometric series of 1 / (1 - e); relative error 2^-65 before rounding)
-__device__ __forceinline__ double rcp_nr(double b) {
-  if (!mid_range(b)) return 1.0 / b;
-  const double x = rcp_seed(b), e = fma_rn(-b, x, 1.0);
-  return fma_rn(x, fma_rn(e, e, e), x);
-}
+// the column pivots' reciprocal in the contracting build.  Without inv_rn's last
+// correction it is two operations shorter but rounds one reciprocal in some
+// thousands the other way than 1 / b (column solve at 256 x 256 x 60 5.74 ms per
+// step, 5.99 now; 100 x 100 x 30 0.754, 0.785).
+__device__ __forceinline__ double pivot_rcp(double b) { return inv_rn(b); }
 // pai^3.5 = pai^3 sqrt(pai), the root by the coupled iteration for g =
 // sqrt(a), h = 1 / (2 sqrt(a)) (Goldschmidt's, as in Markstein's book) from an
 // FP32 estimate and a last correction g + (a - g^2) h: nine FP64 operations
@@ -743,17 +741,17 @@ __device__ __forceinline__ void b_sound_column_std(const View<T>& d, const int j
   if (last) S[(size_t)kz * pl] = T(0);
 }
 
-// The same in the contracting FP64 build, in 38 FP64 operations a level
+// The same in the contracting FP64 build, in 40 FP64 operations a level
 // (about 80 as above).  A = zrom1w dtrdz and B = rdrcv A scale the pressure
 // and divergence differences, and zu, zd = B fzd(k-1) pai(k-1), B fzd(k)
 // pai(k) with the level's products carried to the next.  The pivots run on
 // the complement c = 1 - wwkw (den = (1 + zd c(k+1)) + zu), their reciprocal
-// by rcp_nr.  The moist factors of the Exner/theta update do not change
+// by pivot_rcp.  The moist factors of the Exner/theta update do not change
 // within a sound() call: the first substep forms and stores them (mo1, mo2),
 // the others read those two instead of qv, qc, qwltot, qwitot and divide no
 // more.  The latent-heat branch compares w > 0.1 as integers (positive
 // doubles order as their bits) before it forms anything.
-// 256 x 256 x 60: 8.6 -> 5.1 ms per step (84 % of the FP64 pipe).
+// 256 x 256 x 60: 8.6 -> 6.0 ms per step.
 template <int PD>
 __device__ __forceinline__ void b_sound_column_lean(const View<double>& d, const int jj, const int ii, int nsound,
                                                     int last, int defer_pai) {
@@ -822,7 +820,7 @@ __device__ __forceinline__ void b_sound_column_lean(const View<double>& d, const
     const double ex = fma_rn(B, sub_rn(pzm, pz), sub_rn(fma_rn(-A, sub_rn(x.pkm, pk), x.wk), egdts));
     const double zu = mul_rn(B, fpm), zd = mul_rn(B, fp);
     const double tt = fma_rn(zd, cwp1, 1.0);
-    const double r = rcp_nr(add_rn(tt, zu));
+    const double r = pivot_rcp(add_rn(tt, zu));
     wkp1 = mul_rn(r, fma_rn(zd, wkp1, ex));
     cwp1 = mul_rn(r, tt);
     WPs[o] = wkp1;
@@ -921,9 +919,9 @@ __global__ void __launch_bounds__(kColBX* kColBY, sizeof(T) == 4 && PD == 1 ? 9 
 // right-hand sides and coefficients of all levels side by side, C of them run
 // the recurrence down and the substitution up through shared memory, then all
 // of them update Exner function, theta and pai.  Same expressions and bits as
-// the march, where 10,000 columns are two warps an SM and each level's 38
+// the march, where 10,000 columns are two warps an SM and each level's 40
 // (exact: about 80) FP64 operations, 16 clocks each, wait for the one before.
-// Here only the recurrence (9 and about 18) does, and neither wp nor wwkw leave
+// Here only the recurrence (11 and about 18) does, and neither wp nor wwkw leave
 // the SM.  64 registers, so that four blocks an SM overlap their phases (142
 // registers, one block: 76 us instead of 50 at 100 x 100 x 30).
 constexpr int kSplitThreads = 256;
@@ -1003,7 +1001,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4)
     for (int kk = kz - 1; kk >= 1; --kk) {
       const double ex = sx[kk * C + col], zu = su[kk * C + col], zd = sd[kk * C + col];
       if constexpr (kLean<double>) {
-        const double tt = fma_rn(zd, cwp1, 1.0), r = rcp_nr(add_rn(tt, zu));
+        const double tt = fma_rn(zd, cwp1, 1.0), r = pivot_rcp(add_rn(tt, zu));
         wkp1 = mul_rn(r, fma_rn(zd, wkp1, ex));
         cwp1 = mul_rn(r, tt);
         wwp1 = mul_rn(r, zu);

@@ -223,7 +223,8 @@ int moloch_gpu_check_division_f64(const double* a, const double* b, double* q_nr
  * out themselves, beside CUDA's own (ref), for n device values:
  *   op 0  the quotient a / b from a shared reciprocal (exact build's WAF
  *         values and one-field advection) against a / b;
- *   op 1  the reciprocal 1 / b there.
+ *   op 1  the reciprocal 1 / b there;
+ *   op 2  the reciprocal 1 / b of the contracting build's column pivots.
  * No reference counterpart. */
 int moloch_gpu_check_math_f64(int op, const double* a, const double* b, double* out, double* ref, int n,
                               void* stream);

@@ -1,12 +1,12 @@
 """The FP64 operations the kernels write out themselves, against CUDA's.
 
 Quotients and reciprocals -- the diagnostics' and the moist factors' (the
-contracting build), the shared-reciprocal quotient of the exact build's WAF
-values and of the one-field advection -- round as IEEE: the same bits (any NaN
-for a NaN) on seeded values, on denominators with mantissas on both sides of
-the cut below 2 where the short form ends, numerators beside multiples of
-them, the ends of the exponent ranges, zeros of both signs, subnormals,
-infinities and NaN.
+contracting build), the column pivots' reciprocal, the shared-reciprocal
+quotient of the exact build's WAF values and of the one-field advection --
+round as IEEE: the same bits (any NaN for a NaN) on seeded values, on
+denominators with mantissas on both sides of the cut below 2 where the short
+form ends, numerators beside multiples of them, the ends of the exponent
+ranges, zeros of both signs, subnormals, infinities and NaN.
 """
 import ctypes
 
@@ -15,7 +15,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-QUOT, INV = range(2)
+QUOT, INV, PIVOT = range(3)
 
 
 def check(dm, op, a, b):
@@ -95,7 +95,7 @@ def test_quotients_of_zeros_infinities_and_nan(gpu_lib, op):
     assert same_bits(x, y).all(), report(x, y, a, b)
 
 
-@pytest.mark.parametrize("op", [INV])
+@pytest.mark.parametrize("op", [INV, PIVOT])
 def test_reciprocals_round_as_ieee(gpu_lib, op):
     r = np.random.default_rng(34)
     n = 1 << 21
