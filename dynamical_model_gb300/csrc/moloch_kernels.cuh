@@ -279,11 +279,14 @@ __device__ __forceinline__ double inv_rn(double b) {
 __device__ __forceinline__ double pivot_rcp(double b) { return inv_rn(b); }
 // pai^3.5 = pai^3 sqrt(pai), the root by the coupled iteration for g =
 // sqrt(a), h = 1 / (2 sqrt(a)) (Goldschmidt's, as in Markstein's book) from an
-// FP32 estimate and a last correction g + (a - g^2) h: nine FP64 operations
-// where pow takes about seventy (256 x 256 x 60, with quot_rn: k_prediag 0.93 ->
-// 0.33 ms, k_postdiag 1.14 -> 0.42 ms)
+// FP32 estimate.  The root, its square's residual times h, the cube and the
+// product are each carried in two words (products by the fused residual, T. J.
+// Dekker, Numer. Math. 18, 1971), whose neglected terms are below 2^-80 of the
+// value: half an ulp, where three rounded products reach 2.5 and pow 1.2 ulp.
+// 16 FP64 operations where pow takes about seventy (256 x 256 x 60: k_prediag
+// 0.93 -> 0.42 ms, k_postdiag 1.14 -> 0.47 ms).
 __device__ __forceinline__ double pow35(double a) {
-  static_assert(kCpovr - 3.5 < 1e-15 && 3.5 - kCpovr < 1e-15, "cp / R");
+  static_assert(kCpovr == 3.5, "cp / R");
   if (!mid_range(a) || __double2hiint(a) < 0) return pow(a, kCpovr);
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(narrow_trunc(a)));
@@ -291,8 +294,11 @@ __device__ __forceinline__ double pow35(double a) {
   const double e = fma_rn(-g, h, 0.5);
   g = fma_rn(g, e, g);
   h = fma_rn(h, e, h);
-  g = fma_rn(fma_rn(-g, g, a), h, g);
-  return mul_rn(mul_rn(mul_rn(a, a), a), g);
+  const double gl = mul_rn(fma_rn(-g, g, a), h);  // sqrt(a) - g
+  const double s = mul_rn(a, a), c = mul_rn(s, a);
+  const double cl = fma_rn(fma_rn(a, a, -s), a, fma_rn(s, a, -c));  // a^3 - c
+  const double p = mul_rn(c, g);
+  return add_rn(p, fma_rn(c, gl, fma_rn(cl, g, fma_rn(c, g, -p))));
 }
 #if defined(MOLOCH_LEAN_FP64)
 __device__ __forceinline__ double qdiv(double a, double b) { return quot_rn(a, rcp_rn_of(b)); }

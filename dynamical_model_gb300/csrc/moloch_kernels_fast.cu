@@ -125,7 +125,8 @@ __global__ void k_check_math_f64(int op, const double* __restrict__ a, const dou
     switch (op) {
       case 0: out[q] = quot_rn(x, rcp_rn_of(y)); ref[q] = x / y; break;
       case 1: out[q] = inv_rn(y); ref[q] = 1.0 / y; break;
-      default: out[q] = pivot_rcp(y); ref[q] = 1.0 / y; break;
+      case 2: out[q] = pivot_rcp(y); ref[q] = 1.0 / y; break;
+      default: out[q] = pow_cpovr(x); ref[q] = pow(x, kCpovr); break;
     }
   }
 }
@@ -152,7 +153,7 @@ extern "C" int moloch_gpu_check_division_f64(const double* a, const double* b, d
 }
 extern "C" int moloch_gpu_check_math_f64(int op, const double* a, const double* b, double* out, double* ref, int n,
                                          void* stream) {
-  if (op < 0 || op > 2 || !a || !b || !out || !ref || n < 0) return MOLOCH_ERR_ARG;
+  if (op < 0 || op > 3 || !a || !b || !out || !ref || n < 0) return MOLOCH_ERR_ARG;
   if (n == 0) return MOLOCH_OK;
   const int blocks = (n + 255) / 256 < 1024 ? (n + 255) / 256 : 1024;
   moloch::kfast::k_check_math_f64<<<blocks, 256, 0, (cudaStream_t)stream>>>(op, a, b, out, ref, n);

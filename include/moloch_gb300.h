@@ -224,7 +224,8 @@ int moloch_gpu_check_division_f64(const double* a, const double* b, double* q_nr
  *   op 0  the quotient a / b from a shared reciprocal (exact build's WAF
  *         values and one-field advection) against a / b;
  *   op 1  the reciprocal 1 / b there;
- *   op 2  the reciprocal 1 / b of the contracting build's column pivots.
+ *   op 2  the reciprocal 1 / b of the contracting build's column pivots;
+ *   op 3  a^(cp/R) of the contracting build's diagnostics against pow.
  * No reference counterpart. */
 int moloch_gpu_check_math_f64(int op, const double* a, const double* b, double* out, double* ref, int n,
                               void* stream);

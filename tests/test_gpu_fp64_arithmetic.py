@@ -7,15 +7,22 @@ round as IEEE: the same bits (any NaN for a NaN) on seeded values, on
 denominators with mantissas on both sides of the cut below 2 where the short
 form ends, numerators beside multiples of them, the ends of the exponent
 ranges, zeros of both signs, subnormals, infinities and NaN.
+
+pai^(cp/R): cp/R is 3.5, so the exact value is the square root of an integer
+power, formed here in integers.  pai^3 and the root are carried in two words,
+whose neglected terms lie below 2^-80, so what is left is the last rounding:
+0.5 ulp, and no more than pow's largest error on the same values.
 """
 import ctypes
+import math
 
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-QUOT, INV, PIVOT = range(3)
+QUOT, INV, PIVOT, POW = range(4)
+POW35_ULP = 0.5 + 2.0 ** -20
 
 
 def check(dm, op, a, b):
@@ -102,6 +109,38 @@ def test_reciprocals_round_as_ieee(gpu_lib, op):
     for b in (denominators(), SPECIAL, 1.0 + 10.0 ** r.uniform(-3, 3, n), 2.0 ** r.uniform(-99, 99, n)):
         x, y = check(gpu_lib, op, b, b)
         assert same_bits(x, y).all(), report(x, y, np.ones_like(b), b)
+
+
+def ulps_of_pow35(a, y):
+    """|y - a^3.5| in units of y's last place, from integers"""
+    m, e = math.frexp(a)
+    m, e = int(m * 2 ** 53), 7 * (e - 53)  # a^7 = m^7 2^e
+    k = 400 + (e & 1)
+    s, es = math.isqrt(m ** 7 << k), (e - k) // 2  # a^3.5 = s 2^es
+    my, ey = math.frexp(y)
+    my, ey = int(my * 2 ** 53), ey - 53
+    d = (my << (ey - es)) - s
+    return abs(d) / 2.0 ** (ey - es) if abs(d) < 2 ** 900 else abs(d) // 2 ** (ey - es)
+
+
+@pytest.mark.parametrize("lo,hi", [(0.02, 1.3), (0.95, 1.02), (2.0 ** -99, 2.0 ** 99)])
+def test_exner_power_error(gpu_lib, lo, hi):
+    r = np.random.default_rng(35)
+    n = 20000
+    a = np.exp(r.uniform(math.log(lo), math.log(hi), n))
+    x, y = check(gpu_lib, POW, a, a)
+    ours = max(ulps_of_pow35(float(p), float(q)) for p, q in zip(a, x))
+    cuda = max(ulps_of_pow35(float(p), float(q)) for p, q in zip(a, y))
+    print(f"pai in [{lo:.3g}, {hi:.3g}]: {ours:.6f} ulp, pow {cuda:.6f} ulp")
+    assert ours <= POW35_ULP
+    assert ours <= cuda
+
+
+def test_exner_power_outside_its_range(gpu_lib):
+    a = np.concatenate([SPECIAL, 2.0 ** np.array([-101.0, 101.0, -290.0, 290.0])])
+    x, y = check(gpu_lib, POW, a, a)
+    pow_path = (a <= 0) | ~np.isfinite(a) | (np.abs(a) < 2.0 ** -100) | (np.abs(a) >= 2.0 ** 100)
+    assert same_bits(x, y)[pow_path].all()
 
 
 @pytest.mark.parametrize("plant", [np.inf, -np.inf])
