@@ -841,16 +841,34 @@ int check_launch(const char* what) {
   return MOLOCH_OK;
 }
 
-// reads and clears the flag a bounded device wait sets when it gives up
-int check_kerr(moloch_handle* h) {
-  int* kerr = h->elem == 8 ? h->vd.kerr : h->vf.kerr;
-  int v = 0;
-  CUDA_TRY(cudaMemcpyAsync(&v, kerr, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(cudaStreamSynchronize(h->stream));
+// The flag a bounded device wait sets when it gives up.  watch_kerr copies it
+// to pinned memory in stream order, beside what the caller reads anyway; once
+// that copy has landed, report_kerr turns a set flag into the error and clears
+// it for the steps issued from then on.  (An FP64 handle runs no kernel that
+// waits.)
+int* kerr_of(moloch_handle* h) { return h->elem == 8 ? h->vd.kerr : h->vf.kerr; }
+int watch_kerr(moloch_handle* h) {
+  CUDA_TRY(cudaMemcpyAsync(&h->hres[15], kerr_of(h), sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  return MOLOCH_OK;
+}
+int report_kerr(moloch_handle* h, const void* word) {
+  int v;
+  std::memcpy(&v, word, sizeof v);
   if (!v) return MOLOCH_OK;
-  CUDA_TRY(cudaMemsetAsync(kerr, 0, sizeof(int), h->stream));
-  CUDA_TRY(cudaStreamSynchronize(h->stream));
+  CUDA_TRY(cudaMemsetAsync(kerr_of(h), 0, sizeof(int), h->stream));
   return fail(MOLOCH_ERR_TIMEOUT, "a bounded device wait of the column solve gave up; the state is invalid");
+}
+int check_kerr(moloch_handle* h) {
+  const int rc = watch_kerr(h);
+  if (rc) return rc;
+  CUDA_TRY(cudaStreamSynchronize(h->stream));
+  return report_kerr(h, &h->hres[15]);
+}
+
+// where the output snapshot holds the error flag, behind t and ps
+size_t out_word(const moloch_handle* h) {
+  const size_t pl = (size_t)h->nj() * h->ni();
+  return ((pl * h->kz() + pl) * h->elem + 7) & ~size_t(7);
 }
 
 int read_diag(moloch_handle* h, moloch_diag_t* diag) {
@@ -1166,14 +1184,15 @@ int moloch_gpu_download(moloch_handle_t* h, int field, double* host_base, const 
     return h->elem == 8 ? download_streamed<double>(h, field_ptr(h->vd, f), s, nj, ni, k, level4, host_base)
                         : download_streamed<float>(h, field_ptr(h->vf, f), s, nj, ni, k, level4, host_base);
   };
+  int rc;
+  if (h->elem == 4 && (rc = watch_kerr(h))) return rc;
   if (field == MOLOCH_F_QX) {
-    for (int n = 0; n < 5; ++n) {
-      int rc = down(MOLOCH_F_QV + n, kz, n);
-      if (rc) return rc;
-    }
-    return MOLOCH_OK;
+    for (int n = 0; n < 5; ++n)
+      if ((rc = down(MOLOCH_F_QV + n, kz, n))) return rc;
+  } else if ((rc = down(field, nk, 0))) {
+    return rc;
   }
-  return down(field, nk, 0);
+  return h->elem == 4 ? report_kerr(h, &h->hres[15]) : MOLOCH_OK;
 }
 
 // Output path (the fields the reference driver writes every iout steps,
@@ -1185,7 +1204,7 @@ int moloch_gpu_output_start(moloch_handle_t* h) {
   if (!h || !h->initialized) return fail(MOLOCH_ERR_STATE, "output before moloch_gpu_init");
   if (h->out_pending) return fail(MOLOCH_ERR_STATE, "output_start twice without output_finish");
   const size_t pl = (size_t)h->nj() * h->ni(), n3 = pl * h->kz();
-  const size_t bytes = (n3 + pl) * h->elem;
+  const size_t word = out_word(h), bytes = word + sizeof(int);  // t, ps and the error flag
   if (!h->out_dev) {
     CUDA_TRY(cudaMalloc(&h->out_dev, bytes));
     CUDA_TRY(cudaMallocHost(&h->out_host, bytes));
@@ -1199,6 +1218,7 @@ int moloch_gpu_output_start(moloch_handle_t* h) {
   const void* ps = h->elem == 8 ? (const void*)h->vd.ps : (const void*)h->vf.ps;
   CUDA_TRY(cudaMemcpyAsync(h->out_dev, t, n3 * h->elem, cudaMemcpyDeviceToDevice, h->stream));
   CUDA_TRY(cudaMemcpyAsync((char*)h->out_dev + n3 * h->elem, ps, pl * h->elem, cudaMemcpyDeviceToDevice, h->stream));
+  CUDA_TRY(cudaMemcpyAsync((char*)h->out_dev + word, kerr_of(h), sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
   CUDA_TRY(cudaEventRecord(h->out_taken, h->stream));
   CUDA_TRY(cudaStreamWaitEvent(h->out_stream, h->out_taken, 0));
   CUDA_TRY(cudaMemcpyAsync(h->out_host, h->out_dev, bytes, cudaMemcpyDeviceToHost, h->out_stream));
@@ -1248,7 +1268,7 @@ int moloch_gpu_output_finish(moloch_handle_t* h, double* t_host, const int* t_lb
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(h->out_stream));
     h->out_pending = false;
-    return rc;
+    return rc ? rc : report_kerr(h, (const char*)h->out_host + out_word(h));
   }
   CUDA_TRY(cudaEventSynchronize(h->out_done));
   h->out_pending = false;
@@ -1269,7 +1289,7 @@ int moloch_gpu_output_finish(moloch_handle_t* h, double* t_host, const int* t_lb
   };
   if (t_host) scatter(st, kz, 0, t_host);
   if (ps_host) scatter(sp, 1, n3, ps_host);
-  return MOLOCH_OK;
+  return report_kerr(h, (const char*)h->out_host + out_word(h));
 }
 
 // Idealized initial state computed on the device (param() and

@@ -145,7 +145,9 @@ int moloch_gpu_step(moloch_handle_t* h, int istep, int lprint, moloch_diag_t* di
  * use_graph != 0 replays one CUDA graph of a whole step. */
 int moloch_gpu_run(moloch_handle_t* h, int nsteps, int use_graph);
 
-/* Copy a field back into a reference-layout host array. */
+/* Copy a field back into a reference-layout host array.
+ * MOLOCH_ERR_TIMEOUT (the array is filled all the same) as from
+ * moloch_gpu_sync. */
 int moloch_gpu_download(moloch_handle_t* h, int field, double* host_base,
                         const int* lb, const int* ub);
 
@@ -185,15 +187,20 @@ int moloch_gpu_host_unregister(moloch_handle_t* h, const void* ptr);
  * When both given arrays lie in ranges registered with
  * moloch_gpu_host_register, a kernel on the second stream lays the
  * snapshot out in their Fortran order on the device and the copy engine
- * writes them, instead of host threads. 
- * One snapshot at a time: start, finish, start, ... */
+ * writes them, instead of host threads.
+ * One snapshot at a time: start, finish, start, ...  MOLOCH_ERR_TIMEOUT as
+ * from moloch_gpu_sync when the steps before output_start left the flag set;
+ * the arrays are filled all the same. */
 int moloch_gpu_output_start(moloch_handle_t* h);
 int moloch_gpu_output_finish(moloch_handle_t* h, double* t_host, const int* t_lb, const int* t_ub,
                              double* ps_host, const int* ps_lb, const int* ps_ub);
 
 /* Block until the handle's stream is idle.  MOLOCH_ERR_TIMEOUT when a
  * bounded wait of the staged column kernel gave up since the last check
- * (the state is then invalid); lprint steps check the same flag. */
+ * (the state is then invalid).  lprint steps, moloch_gpu_download and
+ * moloch_gpu_output_finish check the same flag; whichever comes first
+ * reports and clears it.  FP32 handles with jx a multiple of 4 and kz <= 64
+ * start with that kernel. */
 int moloch_gpu_sync(moloch_handle_t* h);
 
 /* Bounded device waits of the staged column kernel (tuning bit 32): every
