@@ -252,6 +252,7 @@ struct moloch_handle {
   // TMA tensor maps of the staged column kernel (FP32 storage), one set per
   // advected-field buffer set
   alignas(64) unsigned char cmaps[4096];
+  bool tuned = false;  // shapes given by the caller or the autotuner; else by default_shapes
   int nj() const { return grid.jx; }
   int ni() const { return grid.iy; }
   int kz() const { return grid.kz; }
@@ -269,11 +270,27 @@ PhaseFlags flags_of(const moloch_handle* h) {
   return f;
 }
 
+// One level, field and tile level a thread: what the slots of a tuning that
+// are not given stand at.  A tuned handle fuses the Coriolis term in the FP32
+// momentum quads and strips (View::cor_rounded).
+template <class T>
+void base_shapes(View<T>& v) {
+  v.hz_levels = 1;
+  v.kmarch = 0;
+  v.vfields = 1;
+  v.srows = kMomR;
+  v.stag4 = 0;
+  v.cor_rounded = 0;
+}
+
 // Launch shapes of a handle nothing else was chosen for (moloch_gpu_set_tuning
-// and moloch_gpu_autotune override them), by the size of the domain.  Every
-// variant named here gives the bits of one level, field and tile level a
-// thread.  us per launch, first the shape up to that size, then the one above
-// it:
+// and moloch_gpu_autotune start again from base_shapes), by the size of the
+// domain.  In FP32 and in the exact build every variant named here gives the
+// bits of the base shapes.  In FP64 all do but the k-marching divergence and
+// momentum, from 20,000 columns on, which form s and the winds from other sums:
+// after three steps w differs by 6e-13 of itself, deltaw by 8e-12, pai by 2e-16
+// (256 x 256 x 20; bound in the tests 1e-11).
+// us per launch, first the shape up to that size, then the one above it:
 //   FP32, jx a multiple of 4 (quads, staged column solve, 16-byte staggering):
 //     divergence + damping 17 | 11 at 100 x 100 x 30, 48 | 26 at 256 x 256 x 40;
 //     momentum 10 | 8 and 39 | 20; column solve 28 | 26 and 64 | 47
@@ -295,11 +312,7 @@ PhaseFlags flags_of(const moloch_handle* h) {
 template <class T>
 void default_shapes(View<T>& v, int mode) {
   const long cols = (long)v.nj * v.ni, pts = cols * v.kz;
-  v.hz_levels = 1;
-  v.kmarch = 0;
-  v.vfields = 1;
-  v.srows = kMomR;
-  v.stag4 = 0;
+  base_shapes(v);
   v.cor_rounded = 1;
   if (mode == MOLOCH_FP32_MIXED) {
     v.srows = 8;
@@ -1453,6 +1466,14 @@ static const int kStripRowCandidates[4] = {4, 8, 16, 32};
 static const int kVFieldCandidates[4] = {1, 2, 5, 10};
 static bool valid_vfields(int f) { return f == 1 || f == 2 || f == 5 || f == 10; }
 
+// the first tuning of a handle: slots not given stand at the base shapes
+static void tune_from_base(moloch_handle_t* h) {
+  if (h->tuned) return;
+  base_shapes(h->vd);
+  base_shapes(h->vf);
+  h->tuned = true;
+}
+
 int moloch_gpu_tuning_count(void) { return kTuneCount; }
 
 int moloch_gpu_set_tuning(moloch_handle_t* h, const int* choice, int n) {
@@ -1466,12 +1487,9 @@ int moloch_gpu_set_tuning(moloch_handle_t* h, const int* choice, int n) {
   if (n > 3 && (choice[3] < 4 || choice[3] > 64))
     return fail(MOLOCH_ERR_ARG, "rows per momentum strip %d", choice[3]);
   if (n > 4 && (choice[4] < 0 || choice[4] > 1)) return fail(MOLOCH_ERR_ARG, "staggering variant %d", choice[4]);
+  tune_from_base(h);
   if (n > 0) { h->vd.hz_levels = choice[0]; h->vf.hz_levels = choice[0]; }
-  if (n > 1) {
-    h->vd.kmarch = choice[1];
-    h->vf.kmarch = choice[1];
-    h->vd.cor_rounded = h->vf.cor_rounded = 0;
-  }
+  if (n > 1) { h->vd.kmarch = choice[1]; h->vf.kmarch = choice[1]; }
   if (n > 2) { h->vd.vfields = choice[2]; h->vf.vfields = choice[2]; }
   if (n > 3) { h->vd.srows = choice[3]; h->vf.srows = choice[3]; }
   if (n > 4) { h->vd.stag4 = choice[4]; h->vf.stag4 = choice[4]; }
@@ -1491,6 +1509,7 @@ int moloch_gpu_autotune(moloch_handle_t* h, int* choice, double* best_ms, int n)
   cudaEvent_t e0, e1;
   CUDA_TRY(cudaEventCreate(&e0));
   CUDA_TRY(cudaEventCreate(&e1));
+  tune_from_base(h);
   double best = 1e30;
   int pick = h->elem == 8 ? h->vd.hz_levels : h->vf.hz_levels;
   for (int c = 0; c < 7; ++c) {

@@ -129,7 +129,8 @@ struct View {
   int srows;       // rows per warp strip of the momentum strips
   int stag4;       // 1: k_stag_from_x4 (FP32, jx a multiple of 4)
   int cor_rounded; // FP32 momentum quads and strips: 1 rounds the Coriolis terms before they are added,
-                   // so that the default shapes give k_sound_momentum's bits; 0 contracts them
+                   // so that the default shapes give k_sound_momentum's bits (untuned handles and
+                   // ensembles); 0 contracts them
 
   // set when a learned surrogate stands in for sound(): the plain sound
   // kernels return at once while *sur_skip == 1 (the surrogate's cycle was

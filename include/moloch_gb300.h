@@ -295,7 +295,18 @@ const char* moloch_gpu_kernel_name(int kind);
  *               columns per thread and 16-byte loads and stores (FP32
  *               storage, jx a multiple of 4; elsewhere, and in ensembles,
  *               ignored), 0: one column per thread.
- * A handle starts with shapes chosen by its size and mode.
+ * A handle or ensemble starts with shapes chosen by its size and mode.  The
+ * first set_tuning (of any number of slots) or autotune starts again from one
+ * level, field and tile level a thread, [1, 0, 1, 32, 0] (ensembles [4, 0, 1,
+ * 32, 0]): slots not given stand there.  It also decides one rounding: the
+ * FP32 momentum variants of bits 8 and 64 add the Coriolis term by a fused
+ * multiply-add on a tuned handle, and round its product first, as the
+ * one-level kernel does, on an untuned one -- so an untuned handle's results
+ * do not depend on its size, a tuned handle's are those of the tuning, and
+ * giving a handle the shapes it already runs moves u and v by a rounding.  In
+ * MOLOCH_FP64 the k-marching divergence and momentum (bits 1 and 4, and
+ * untuned handles from 20,000 columns or ensembles from 2^20 points on) round
+ * differently from the one-level kernels.
  * moloch_gpu_autotune runs advection() and sound() once per candidate and
  * repeat, so it advances the model state: call it on a scratch handle or before the
  * initial state is uploaded again.  The chosen values can be cached by the
