@@ -355,9 +355,22 @@ size_t layout(View<T>& v, char* base, const moloch_handle* h) {
   v.p = T3(); v.qsat = T3(); v.tvirt = T3(); v.rho = T3(); v.ps = T2();
   v.qwltot = T3(); v.qwitot = T3();
   v.s = T3p(); v.deltaw = T3p(); v.zdiv2a = T3(); v.zdiv2b = T3();
-  v.wp = (double*)take(sizeof(double) * n3p);
-  v.wwkw = (double*)take(sizeof(double) * n3p);
   v.wz = (T*)take(sizeof(T) * n3 * kNumAdvected);
+  // MOLOCH_FP64 has more static terms than the other modes (fzd, which takes
+  // the place of fmz, and fmx) and two fields of a sound() call (mo1, mo2).  It
+  // keeps to their memory: what only lives within a sound() call lies in wz,
+  // which advection() writes before it reads.
+  const bool lean = h->prm.mode == MOLOCH_FP64;
+  v.mo1 = v.mo2 = nullptr;
+  if (lean) {
+    v.wp = (double*)v.wz;
+    v.wwkw = base ? v.wp + n3p : nullptr;
+    v.mo1 = base ? v.wz + 2 * n3p : nullptr;
+    v.mo2 = base ? v.mo1 + n3 : nullptr;
+  } else {
+    v.wp = (double*)take(sizeof(double) * n3p);
+    v.wwkw = (double*)take(sizeof(double) * n3p);
+  }
   const bool filt = h->prm.do_filterpai || h->prm.do_filtertheta;
   v.pf = h->prm.do_filterpai ? T3() : nullptr;
   v.tf = h->prm.do_filtertheta ? T3() : nullptr;
@@ -365,9 +378,8 @@ size_t layout(View<T>& v, char* base, const moloch_handle* h) {
   v.eu_j = T1(ne); v.eu_i = T1(ne); v.ev_j = T1(ne); v.ev_i = T1(ne); v.ep_j = T1(ne); v.ep_i = T1(ne);
   v.fmz = T3(); v.fmzf = T3p(); v.zeta = T3(); v.dz = T3();
   v.rfw = T3(); v.rfs = T3();
-  v.fmx = v.fzd = nullptr;
-  v.mo1 = v.mo2 = nullptr;
-  if (h->prm.mode == MOLOCH_FP64) { v.fmx = T3(); v.fzd = T3(); v.mo1 = T3(); v.mo2 = T3(); }
+  v.fmx = lean ? T3() : nullptr;
+  v.fzd = lean ? v.fmz : nullptr;
   v.wafu = T3(); v.wafd = T3(); v.wafn = T3(); v.wafs = T3(); v.wafe = T3(); v.wafw = T3();
   v.hx = T2(); v.hy = T2(); v.mx = T2(); v.mu = T2(); v.mv = T2(); v.rmu = T2(); v.rmv = T2();
   v.mx2 = T2(); v.coru = T2(); v.corv = T2();
@@ -762,13 +774,13 @@ int init_impl(moloch_handle* h, View<T>& v) {
     }
   }, transfer_threads(sizeof(double) * 16 * n3));
   auto up3 = [&](const T* dst, const std::vector<double>& src) { return upload_dense<T>(h, (T*)dst, src); };
-  if ((rc = up3(v.fmz, fmz)) || (rc = up3(v.fmzf, fmzf)) || (rc = up3(v.zeta, h->zeta))) return rc;
+  if ((rc = up3(v.fmz, lean ? fzd : fmz)) || (rc = up3(v.fmzf, fmzf)) || (rc = up3(v.zeta, h->zeta))) return rc;
   if ((rc = up3(v.rfw, rfw)) || (rc = up3(v.rfs, rfs)) || (rc = up3(v.wafu, wu)) || (rc = up3(v.wafd, wd)))
     return rc;
   if ((rc = up3(v.wafn, wn)) || (rc = up3(v.wafs, ws)) || (rc = up3(v.wafe, we)) || (rc = up3(v.wafw, ww)))
     return rc;
   if ((rc = up3(v.dz, dz))) return rc;
-  if (lean && ((rc = up3(v.fmx, fmx)) || (rc = up3(v.fzd, fzd)))) return rc;
+  if (lean && (rc = up3(v.fmx, fmx))) return rc;
   // w(:,:,1) = 0 (:260-262); s, deltaw zero (reset_tendencies :1313-1325 --
   // the kernels never write s(1), deltaw(1), deltaw(kz+1), which therefore
   // keep this zero for the whole run)

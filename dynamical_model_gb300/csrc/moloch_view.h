@@ -51,13 +51,13 @@ struct View {
   T* zdiv2a;  // horizontal divergence (Equation 16)
   T* zdiv2b;  // after divdamp and the vertical s term
   T* mo1;  // moist factors of the Exner/theta update, written by a sound()
-  T* mo2;  // call's first substep and read by the others (kLean)
+  T* mo2;  // call's first substep and read by the others (kLean; with wp and wwkw in wz's memory)
   double* wp;    // Thomas down-sweep values (FP64 in every mode), kz+1 levels
   double* wwkw;  // Thomas pivot ratios (FP64 in every mode), kz+1 levels
   T* ux;
   T* vx;
   T* wx;
-  T* wz;  // kNumAdvected fields (vertical WAF result)
+  T* wz;  // kNumAdvected fields (vertical WAF result); MOLOCH_FP64: also wp, wwkw, mo1 and mo2 within sound()
   // the ten advected fields live in two buffer sets; the horizontal WAF
   // step writes the other set (fset[fcur ^ 1]) and the sets swap roles
   T* fset[2][kNumAdvected];
@@ -74,18 +74,18 @@ struct View {
   T* ep_i;  // pai before its update at i = ni, per (j, k)  [pai(j, 0)]
 
   // static 3-D metric terms (computed once on the host in FP64)
-  const T* fmz;
+  const T* fmz;   // MOLOCH_FP64: fzd
   const T* fmzf;  // kz+1 levels
   const T* zeta;
   const T* dz;
   // rfw, rfs: 2 / (fmz(j) + fmz(j-1)), 2 / (fmz(i) + fmz(i-1)).  MOLOCH_FP64
   // (the contracting FP64 build, kLean) holds every static factor of
-  // Equation 16 in them, dtrdx (rmu) rfw and dtrdy rmv rfs, and has three
-  // more arrays (nullptr elsewhere)
+  // Equation 16 in them, dtrdx (rmu) rfw and dtrdy rmv rfs, and has fmx and
+  // fzd (nullptr elsewhere)
   const T* rfw;
   const T* rfs;
   const T* fmx;   // fmz mx (ROTLLR) or fmz mx2
-  const T* fzd;   // fmz dtrdz
+  const T* fzd;   // fmz dtrdz, in the place of fmz
   const T* wafu;  // wafone zrfmu
   const T* wafd;  // wafone zrfmd
   const T* wafn;  // wafone zrfmn
