@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "moloch_constants.h"
+#include "moloch_device.h"
 #include "moloch_view.h"
 
 #ifndef MOLOCH_KNS
@@ -4098,16 +4099,6 @@ int launch_prediag(const View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
 template <class T>
 inline bool column_tm_ok(const View<T>& d) {
   return sizeof(T) == 4 && (d.kmarch & 32) && d.cmaps != nullptr;
-}
-inline int sm_count() {
-  static int nsm = 0;
-  if (!nsm) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (nsm <= 0) nsm = 1;
-  }
-  return nsm;
 }
 // the one-thread column solve (variants: k_sound_column)
 template <class T>
