@@ -54,7 +54,8 @@ ALG_WORDS = {
     "k_sound_damp": 8,        # r: zdiv2a u v fmz s | w: u v zdiv2b
     "k_sound_divdamp": 9,     # r: u v fmz rfw rfs | w: u v s zdiv2b (fused div + damp)
     "k_sound_column": 16,     # r: w fmzf qv tetav pai qsat t zdiv2b fmz qc qwltot qwitot | w: w deltaw tetav pai
-    "k_sound_column_tm": 16,  # the same arrays (the TMA-staged column solve)
+    "k_sound_column_tw": 16,  # the same arrays (the TMA-staged column solve)
+    "k_sound_column_tm": 16,  # its name in earlier result lines
     "k_sound_momentum": 7,    # r: u v deltaw tetav pai | w: u v
     "k_waf_vertical": 26,     # r: 7 fields u v w s wafu wafd | w: 10 wz ux vx wx
     "k_waf_horizontal": 36,   # r: 10 wz 10 pp u v wafn wafs wafe wafw | w: 10 pp
@@ -66,24 +67,26 @@ ALG_WORDS = {
 # scaled by the point count to the benchmarked size (traffic grows in
 # proportion: one pass over each array per launch)
 _STAGED = (1055.7e6, 512 * 512 * 60)
-NCU_TRAFFIC = {"k_sound_column": (847.0e6, 384 * 384 * 60), "k_sound_column_tm": _STAGED,
-               "k_sound_column_tw12": _STAGED}
+NCU_TRAFFIC = {"k_sound_column": (847.0e6, 384 * 384 * 60), "k_sound_column_tw": _STAGED}
 # sm__pipe_fp64_cycles_active (% of peak, active) from the same captures
+_STAGED_PIPE = {"pipe_fp64_active_pct": 53.9, "capture": "512x512x60", "fp64_operations_per_level": 4}
 NCU_FP64_PIPE = {"k_sound_column": {"pipe_fp64_active_pct": 35.7, "capture": "384x384x60",
                                     "fp64_operations_per_level": 4},
-                 "k_sound_column_tm": {"pipe_fp64_active_pct": 53.9, "capture": "512x512x60",
-                                       "fp64_operations_per_level": 4},
-                 "k_sound_column_tw12": {"pipe_fp64_active_pct": 53.9, "capture": "512x512x60",
-                                         "fp64_operations_per_level": 4}}
+                 "k_sound_column_tw": _STAGED_PIPE}
+# the names earlier result lines gave the staged column solve, once three kernels
+for _name in ("k_sound_column_tm", "k_sound_column_tw12"):
+    NCU_TRAFFIC[_name], NCU_FP64_PIPE[_name] = _STAGED, _STAGED_PIPE
 
 
 def column_variant(name, tuning):
-    """Name of the staged column solve under the profile's kernel kind
-    k_sound_column_tm, by the tuning's bits; all of them run the same kernel
-    (two words of column state a level, two CTAs an SM)."""
+    """Name an earlier result line gives the staged column solve, whose
+    profile kind was k_sound_column_tm, under a tuning: for reading those
+    lines.  Profiles now name the one kernel there is, k_sound_column_tw."""
     if name != "k_sound_column_tm" or len(tuning) < 2:
         return name
     return "k_sound_column_tw12" if tuning[1] & 128 else "k_sound_column_tw16" if tuning[1] & 256 else name
+
+
 # the FP64 step's kernels are bound by GB300's FP64 rate, not HBM: their
 # FP64-pipe activity from one-launch ncu captures at 256x256x60
 NCU_FP64_STEP = {"k_sound_column": {"pipe_fp64_active_pct": 83.3, "dram_pct": 20.3},
@@ -663,22 +666,21 @@ def run_single(args, dist, rank, ws, torch, dm, stream, local, device):
     peak, peak_kind = peaks()
     top = max(prof.items(), key=lambda kv: kv[1][0])
     tkind, (tms, tcount) = top
-    tname = column_variant(tkind, tune_mix)
     words = ALG_WORDS.get(tkind, 0)
     esz = 4
     alg_bytes = words * esz * gp  # per launch
     avg_ms = tms / max(tcount, 1)
     achieved = alg_bytes / (avg_ms / 1e3) / 1e9
-    roofline = {"bound": "hbm", "kernel": tname, "achieved": achieved, "peak": peak,
+    roofline = {"bound": "hbm", "kernel": tkind, "achieved": achieved, "peak": peak,
                 "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                 "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_ms,
-                "traffic": (NCU_TRAFFIC[tname][0] * gp / NCU_TRAFFIC[tname][1]) if tname in NCU_TRAFFIC else None,
+                "traffic": (NCU_TRAFFIC[tkind][0] * gp / NCU_TRAFFIC[tkind][1]) if tkind in NCU_TRAFFIC else None,
                 "traffic_note": "ncu dram bytes of one launch (512x512x60; the one-thread solve 384x384x60), scaled "
                                 "by grid points (part of the writes is still in L2 when it ends)",
                 # second roof of the top kernel: its FP64 pivot recurrence (4
                 # FP64 operations per level) keeps the FP64 pipe this busy in
                 # the ncu capture of the same kernel
-                "fp64_pipe": NCU_FP64_PIPE.get(tname),
+                "fp64_pipe": NCU_FP64_PIPE.get(tkind),
                 "step_alg_GBps": B_ALG_WORDS * esz * value_mix / n_dom / 1e9}
     kernels = {k: {"ms": round(v[0], 4), "launches": v[1],
                    "GBps_alg": (ALG_WORDS.get(k, 0) * esz * gp * v[1] / (v[0] / 1e3) / 1e9) if v[0] > 0 else None}

@@ -4097,7 +4097,7 @@ int launch_prediag(const View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
 // the staged column kernel runs when asked for (kmarch bit 32) on an FP32
 // domain whose tensor maps were built
 template <class T>
-inline bool column_tm_ok(const View<T>& d) {
+inline bool column_tw_ok(const View<T>& d) {
   return sizeof(T) == 4 && (d.kmarch & 32) && d.cmaps != nullptr;
 }
 // the one-thread column solve (variants: k_sound_column)
@@ -4207,14 +4207,14 @@ int launch_sound(View<T>& d, cudaStream_t st, const PhaseFlags& fl) {
     } else {
       bool staged = false;
       if constexpr (sizeof(T) == 4) {
-        if (column_tm_ok(d)) {
+        if (column_tw_ok(d)) {
           const ColumnMaps& cm = static_cast<const ColumnMaps*>(d.cmaps)[d.fcur];
           const int grid = column_tw_grid(d);
           if (last)
-            MOLOCH_LAUNCH(KK_SOUND_COLUMN_TM, st,
+            MOLOCH_LAUNCH(KK_SOUND_COLUMN_TW, st,
                           k_sound_column_tw<T, 1><<<grid, TwCfg<1>::threads, TwCfg<1>::smem, st>>>(d, cm, ns));
           else
-            MOLOCH_LAUNCH(KK_SOUND_COLUMN_TM, st,
+            MOLOCH_LAUNCH(KK_SOUND_COLUMN_TW, st,
                           k_sound_column_tw<T, 0><<<grid, TwCfg<0>::threads, TwCfg<0>::smem, st>>>(d, cm, ns));
           staged = true;
         }
