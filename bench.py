@@ -88,13 +88,15 @@ def column_variant(name, tuning):
 
 
 # the FP64 step's kernels are bound by GB300's FP64 rate, not HBM: their
-# FP64-pipe activity from one-launch ncu captures at 256x256x60
-NCU_FP64_STEP = {"k_sound_column": {"pipe_fp64_active_pct": 83.3, "dram_pct": 20.3},
-                 "k_waf_vertical": {"pipe_fp64_active_pct": 71.7, "dram_pct": 7.1},
-                 "k_waf_horizontal": {"pipe_fp64_active_pct": 75.4, "dram_pct": 8.8},
-                 "k_sound_momentum": {"pipe_fp64_active_pct": 77.5, "dram_pct": 10.6},
-                 "k_sound_div": {"pipe_fp64_active_pct": 86.4, "dram_pct": 21.0},
-                 "k_sound_damp": {"pipe_fp64_active_pct": 85.9, "dram_pct": 26.8}}
+# FP64-pipe activity from one-launch ncu captures at 256x256x60, in the shapes
+# a handle of that size starts with (strips of 32 rows, k-marching, five fields
+# a thread), which the autotuner picks as well
+NCU_FP64_STEP = {"k_sound_column": {"pipe_fp64_active_pct": 84.5, "dram_pct": 20.7},
+                 "k_waf_vertical": {"pipe_fp64_active_pct": 78.7, "dram_pct": 7.3},
+                 "k_waf_horizontal": {"pipe_fp64_active_pct": 87.6, "dram_pct": 12.2},
+                 "k_sound_momentum": {"pipe_fp64_active_pct": 76.9, "dram_pct": 10.6},
+                 "k_sound_div": {"pipe_fp64_active_pct": 86.9, "dram_pct": 23.1},
+                 "k_sound_damp": {"pipe_fp64_active_pct": 85.1, "dram_pct": 26.7}}
 # whole-step algorithmic words per grid point of the fused design target
 # (pre-diag 11 + 3 sound cycles x 91 + 3 advection steps x 23 + post-diag 11)
 B_ALG_WORDS = 364

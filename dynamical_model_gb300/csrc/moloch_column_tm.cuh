@@ -455,8 +455,8 @@ __global__ void __launch_bounds__(TwCfg<LAST>::threads, TwCfg<LAST>::ctas)
 
 // An ensemble's column tiles in one persistent launch: the tile table
 // lists (member, tile x, tile y) heaviest member first; cms holds each
-// member's tensor maps for the 12-row boxes, two buffer-set parities per
-// member.  A wait that gives up sets *kerr (the ensemble's error word).
+// member's tensor maps, whose boxes have its tiles' shape (View::twide), two
+// buffer-set parities per member.  A wait that gives up sets *kerr (the ensemble's error word).
 template <class T, int LAST>
 __global__ void __launch_bounds__(TwCfg<LAST>::threads, TwCfg<LAST>::ctas)
     kb_sound_column_tw(const View<T>* __restrict__ views, const ColumnMaps* __restrict__ cms,

@@ -564,10 +564,10 @@ __device__ __forceinline__ T zrom1w_moist(T zrom1w, T qvk, T qsk, T qskm, T wk, 
 // with the Exner/theta/pai update of the level above it.
 // defer_pai: leave zdiv2b final and pai to k_pai_update (divergence filter on).
 // PD: levels loaded ahead of the level computed, in both sweeps (a register
-// ring of PD level records).  The kernels use PD = 1.  A ring of 3 levels at 4 blocks per SM (so
-// that the back-substitution finds more of the down-sweep's levels in L2)
-// measured 13 % slower at 512 x 512 x 60: fewer columns in flight cost more
-// bandwidth than the extra L2 hits saved.
+// ring of PD level records): 1, and 2 on small FP32 grids (k_sound_column).  A
+// ring of 3 levels at 4 blocks per SM (so that the back-substitution finds more
+// of the down-sweep's levels in L2) measured 13 % slower at 512 x 512 x 60:
+// fewer columns in flight cost more bandwidth than the extra L2 hits saved.
 template <class T, int PD>
 __device__ __forceinline__ void b_sound_column_std(const View<T>& d, const int jj, const int ii, int nsound, int last, int defer_pai) {
   const int nj = d.nj, ni = d.ni, kz = d.kz;
@@ -748,7 +748,7 @@ __device__ __forceinline__ void b_sound_column_std(const View<T>& d, const int j
   if (last) S[(size_t)kz * pl] = T(0);
 }
 
-// The same in the contracting FP64 build, in 40 FP64 operations a level
+// The same in the contracting FP64 build, in 39 FP64 operations a level
 // (about 80 as above).  A = zrom1w dtrdz and B = rdrcv A scale the pressure
 // and divergence differences, and zu, zd = B fzd(k-1) pai(k-1), B fzd(k)
 // pai(k) with the level's products carried to the next.  The pivots run on
@@ -757,7 +757,8 @@ __device__ __forceinline__ void b_sound_column_std(const View<T>& d, const int j
 // within a sound() call: the first substep forms and stores them (mo1, mo2),
 // the others read those two instead of qv, qc, qwltot, qwitot and divide no
 // more.  The latent-heat branch compares w > 0.1 as integers (positive
-// doubles order as their bits) before it forms anything.
+// doubles order as their bits) before it forms anything.  It leaves out the
+// ffilt(k) the other solves add to zu and zd, which is zero (View::ffilt).
 // 256 x 256 x 60: 8.6 -> 6.0 ms per step.
 template <int PD>
 __device__ __forceinline__ void b_sound_column_lean(const View<double>& d, const int jj, const int ii, int nsound,
@@ -926,11 +927,12 @@ __global__ void __launch_bounds__(kColBX* kColBY, sizeof(T) == 4 && PD == 1 ? 9 
 // right-hand sides and coefficients of all levels side by side, C of them run
 // the recurrence down and the substitution up through shared memory, then all
 // of them update Exner function, theta and pai.  Same expressions and bits as
-// the march, where 10,000 columns are two warps an SM and each level's 40
+// the march, where 10,000 columns are two warps an SM and each level's 39
 // (exact: about 80) FP64 operations, 16 clocks each, wait for the one before.
 // Here only the recurrence (11 and about 18) does, and neither wp nor wwkw leave
 // the SM.  64 registers, so that four blocks an SM overlap their phases (142
-// registers, one block: 76 us instead of 50 at 100 x 100 x 30).
+// registers, one block: 76 us instead of 50 at 100 x 100 x 30, with a reciprocal
+// of two operations less).
 constexpr int kSplitThreads = 256;
 constexpr size_t split_smem_bytes(int columns, int kz) { return (size_t)3 * kz * columns * sizeof(double); }
 template <int C>
@@ -4106,12 +4108,20 @@ void launch_sound_column(const View<T>& d, cudaStream_t st, int ns, int last, in
   if constexpr (sizeof(T) == 8) {
     // FP64 columns split over a block (k_sound_column_split) while the march
     // leaves SMs idle.  us per launch, march | 32 columns a block | 8:
-    //   lean   35 | 17 | 14 at 24 x 20 x 12, 55 | 25 | 22 at 53 x 47 x 21, 74 | 33 | 32
-    //          at 64 x 64 x 30, 79 | 50 | 72 at 100 x 100 x 30, 163 | 148 | 250 at
-    //          203 x 157 x 45, 365 | 372 | 659 at 256 x 256 x 60
+    //   lean   37 | 19 | 15 at 24 x 20 x 12, 57 | 26 | 24 at 53 x 47 x 21, 77 | 35 | 35
+    //          at 64 x 64 x 30, 81 | 53 | 78 at 100 x 100 x 30, 170 | 154 | 273 at
+    //          203 x 157 x 45, 304 | 269 | 458 at 199 x 200 x 60, 386 | 392 | 716 at
+    //          256 x 256 x 60
     //   exact  47 | 23 | 16, 74 | 34 | 31, 104 | 46 | 47, 104 | 82 | 106; 170 | 178 |
     //          240 at 150 x 140 x 40
-    // Deeper columns take fewer to a block (48 KB of shared memory).
+    // Deeper columns take fewer to a block (48 KB of shared memory), march | 16
+    // columns a block | 8:
+    //   lean   178 | 60 | 52 at 24 x 20 x 72, 181 | 66 | 64 at 53 x 47 x 72, 325 | 120 |
+    //          111 at 54 x 55 x 128, 205 | 166 | 241 at 126 x 126 x 72, 362 | 289 | 422
+    //          at 126 x 126 x 128, 286 | 305 | 434 at 160 x 160 x 96; 729 | - | 205 at
+    //          53 x 47 x 256
+    //   exact  243 | 76 | 62, 239 | 93 | 84, 419 | 167 | 147, 254 | 255 | 337, 445 | 445 |
+    //          591, 463 | 509 | 678; 832 | - | 279
     const auto split = [&](auto k, int cols) {
       MOLOCH_LAUNCH(KK_SOUND_COLUMN, st,
                     k<<<((unsigned)d.pl + cols - 1) / cols, kSplitThreads, split_smem_bytes(cols, d.kz), st>>>(d, ns, last,

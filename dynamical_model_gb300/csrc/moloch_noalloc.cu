@@ -294,7 +294,7 @@ extern "C" int moloch_gpu_wafone_noalloc(double* pp, const double* s, const doub
     moloch_internal_set_error("wafone_noalloc: jx, iy and kz must be >= 4");
     return MOLOCH_ERR_ARG;
   }
-  if (kz > 65535) {  // the meridional and zonal kernels take k as gridDim.z
+  if (kz > 65535) {  // the meridional kernel takes k as gridDim.y, the zonal one kz / 2
     moloch_internal_set_error("wafone_noalloc: kz must be <= 65535");
     return MOLOCH_ERR_ARG;
   }

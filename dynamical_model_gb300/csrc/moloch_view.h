@@ -108,7 +108,7 @@ struct View {
   const T* gzitakh;  // kz
   const T* xknu;     // kz
   const T* cdamp;    // xknu(k) * ddamp
-  const T* ffilt;    // kz (zero in the reference)
+  const T* ffilt;    // kz; zero, as in the reference: the MOLOCH_FP64 column solve does not read it
 
   // scalars of sound() (dts) and wafone() (dta)
   T dts, dtrdx, dtrdy, dtrdz, zcs2, ddamp2, egdts;
